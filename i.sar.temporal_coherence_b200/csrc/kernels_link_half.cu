@@ -48,62 +48,92 @@
 
 namespace {
 
-struct Grp {
+/* A half-warp. Collectives take their mask from members(): Pair, for code
+   that both halves of the warp run together, names all 32 lanes, a constant
+   (shuffles, votes and warp barriers with a mask that is only known at run
+   time first make the named lanes meet: on B200 a shuffle takes 52 cycles with
+   such a mask and 37 with a constant one, a warp barrier 23 and 10; the link
+   stage of a 512 x 4096 AD / EMI / -b strip at 30 dates went from 100.2 to
+   94.4 ms, EVD at 250 x 1000 from 7.06 to 6.56); Grp, for
+   branches that one half may take alone (the rare fallback tiers and the
+   refinement), names its own 16. */
+struct Pair {
     int lane, gl, base;
-    unsigned mask;
+
+    __device__ __forceinline__ unsigned members() const { return FULL; }
 };
 
-__device__ __forceinline__ Grp make_grp(int lane)
+struct Grp : Pair {
+    __device__ __forceinline__ unsigned members() const { return 0xFFFFu << base; }
+};
+
+__device__ __forceinline__ Pair make_pair(int lane)
 {
-    Grp g;
+    Pair g;
 
     g.lane = lane;
     g.gl = lane & 15;
     g.base = lane & 16;
-    g.mask = 0xFFFFu << g.base;
     return g;
 }
 
-template <typename T>
-__device__ __forceinline__ T gsum(T v, const Grp &g)
+__device__ __forceinline__ Grp alone(const Pair &p)
+{
+    Grp g;
+
+    g.lane = p.lane;
+    g.gl = p.gl;
+    g.base = p.base;
+    return g;
+}
+
+template <typename T, class G>
+__device__ __forceinline__ T gsum(T v, const G &g)
 {
 #pragma unroll
     for (int o = 8; o; o >>= 1)
-        v += __shfl_xor_sync(g.mask, v, o);
+        v += __shfl_xor_sync(g.members(), v, o);
     return v;
 }
 
-__device__ __forceinline__ float gmaxf(float v, const Grp &g)
+template <class G>
+__device__ __forceinline__ float gmaxf(float v, const G &g)
 {
 #pragma unroll
     for (int o = 8; o; o >>= 1)
-        v = fmaxf(v, __shfl_xor_sync(g.mask, v, o));
+        v = fmaxf(v, __shfl_xor_sync(g.members(), v, o));
     return v;
 }
 
-__device__ __forceinline__ float gminf(float v, const Grp &g)
+template <class G>
+__device__ __forceinline__ float gminf(float v, const G &g)
 {
 #pragma unroll
     for (int o = 8; o; o >>= 1)
-        v = fminf(v, __shfl_xor_sync(g.mask, v, o));
+        v = fminf(v, __shfl_xor_sync(g.members(), v, o));
     return v;
 }
 
-__device__ __forceinline__ double gmaxd(double v, const Grp &g)
+template <class G>
+__device__ __forceinline__ double gmaxd(double v, const G &g)
 {
 #pragma unroll
     for (int o = 8; o; o >>= 1)
-        v = fmax(v, __shfl_xor_sync(g.mask, v, o));
+        v = fmax(v, __shfl_xor_sync(g.members(), v, o));
     return v;
 }
 
-template <typename T>
-__device__ __forceinline__ T gbcast(T v, int row, const Grp &g)
+template <typename T, class G>
+__device__ __forceinline__ T gbcast(T v, int row, const G &g)
 {
-    return __shfl_sync(g.mask, v, g.base | (row & 15));
+    return __shfl_sync(g.members(), v, g.base | (row & 15));
 }
 
-__device__ __forceinline__ void gsync(const Grp &g) { __syncwarp(g.mask); }
+template <class G>
+__device__ __forceinline__ void gsync(const G &g)
+{
+    __syncwarp(g.members());
+}
 
 /* Per-group shared workspace (byte offsets, 16-byte aligned). */
 struct HalfLayout {
@@ -161,7 +191,7 @@ struct StepHead {
     float dk;
 };
 
-__device__ __forceinline__ StepHead step_head(float2 c0, float2 c1, int k, int n, const Grp &g)
+__device__ __forceinline__ StepHead step_head(float2 c0, float2 c1, int k, int n, const Pair &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
     StepHead h;
@@ -191,7 +221,7 @@ __device__ __forceinline__ float2 r2(float2 t, float2 nv, float2 nw, float4 q)
 }
 
 __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs &w, int ld,
-                            const Grp &g)
+                            const Pair &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
 
@@ -343,7 +373,8 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
        x  -= sum_m v_m h_m
    (tau' = conj(tau) for Q^H), which is the sequential application
    rearranged. */
-__device__ void apply_q(int n, int ld, const HWs &w, const Grp &g, bool adjoint, float2 &x0,
+template <class G>
+__device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, float2 &x0,
                         float2 &x1)
 {
     const int i0 = g.gl, i1 = g.gl + 16, nk = n - 1;
@@ -433,7 +464,7 @@ __device__ __forceinline__ int sturm16(const float *d, const float *e2, int n, f
 
 /* Eigenvalue of rank `index` of the group's tridiagonal (w.d, w.e), by
    17-way multisection of its Gershgorin interval. */
-__device__ float tri_eigenvalue(int n, int index, const HWs &w, const Grp &g, float &norm,
+__device__ float tri_eigenvalue(int n, int index, const HWs &w, const Pair &g, float &norm,
                                 unsigned &status)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
@@ -459,40 +490,36 @@ __device__ float tri_eigenvalue(int n, int index, const HWs &w, const Grp &g, fl
     hi += 1.0e-6f * norm + 1.0e-30f;
     gsync(g);
     const float pivmin = 1.0e-30f + 1.0e-14f * norm;
-    int round = 0;
+    /* The two halves of the warp go through the rounds together; one that is
+       done keeps its interval. */
+    bool open = true;
+    int rounds = 0;
 
-    for (; round < 20; round++) {
+    for (int round = 0; round < 20; round++) {
         /* 1e-7 of the spectrum's scale is all that the inverse iteration
            and the solves off the eigenvector need (the eigenvector's
            accuracy comes from those); the smallest eigenvalues of EMI would
            otherwise take several more rounds down to their own ulp */
         if (hi - lo <= 1.0e-7f * norm)
+            open = false;
+        if (!__any_sync(FULL, open))
             break;
         const float xq = lo + (hi - lo) * ((float)(g.gl + 1) * (1.0f / 17.0f));
         const int cnt = sturm16(w.d, w.e2f, n, xq, pivmin);
-        const unsigned gt = (__ballot_sync(g.mask, cnt > index) >> g.base) & 0xFFFFu;
-        float nlo, nhi;
+        const unsigned gt = (__ballot_sync(FULL, cnt > index) >> g.base) & 0xFFFFu;
+        const int f = gt ? __ffs(gt) - 1 : 16;
+        const float xh = gbcast(xq, f & 15, g), xl = gbcast(xq, f > 0 ? f - 1 : 0, g);
+        const float nlo = fmaxf(f > 0 ? xl : lo, lo), nhi = fminf(f < 16 ? xh : hi, hi);
 
-        if (gt == 0u) {
-            nlo = gbcast(xq, 15, g);
-            nhi = hi;
-        }
-        else {
-            const int f = __ffs(gt) - 1;
-
-            nhi = gbcast(xq, f, g);
-            nlo = gbcast(xq, f > 0 ? f - 1 : 0, g);
-            if (f == 0)
-                nlo = lo;
-        }
-        nlo = fmaxf(nlo, lo);
-        nhi = fminf(nhi, hi);
         if (!(nlo > lo || nhi < hi))
-            break;
-        lo = nlo;
-        hi = nhi;
+            open = false;
+        if (open) {
+            lo = nlo;
+            hi = nhi;
+            rounds++;
+        }
     }
-    if (round == 20)
+    if (rounds == 20)
         status |= TC_STATUS_ITER_CAP;
     return 0.5f * (lo + hi);
 }
@@ -504,7 +531,7 @@ __device__ __forceinline__ float rcpx(float x) { return __fdividef(1.0f, x); }
 /* Partially pivoted LU of tri - lambda I, into w.lu (written by the first
    lane of the group); returns the pivot bits. Every lane computes it. */
 template <typename R>
-__device__ unsigned long long tri_lu(int n, R lambda, R tiny, const HWs &w, const Grp &g)
+__device__ unsigned long long tri_lu(int n, R lambda, R tiny, const HWs &w, const Pair &g)
 {
     R dd = (R)w.d[0] - lambda, s1 = n > 1 ? (R)w.e[0] : (R)0;
     unsigned long long piv = 0ull;
@@ -577,7 +604,7 @@ __device__ __forceinline__ void tri_solve(float (&yr)[32], int n, unsigned long 
 /* The eigenvector of rank `index` of the reduced matrix, back-transformed:
    returns the components of rows i0, i1 in z0, z1; y (tridiagonal vector)
    is left in yr. */
-__device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Grp &g, float2 &z0,
+__device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g, float2 &z0,
                            float2 &z1, float (&yr)[32], float &lambda, float &norm,
                            unsigned long long &piv)
 {
@@ -654,10 +681,12 @@ __device__ __forceinline__ double rcp_newton(double d)
    register column p holds true column (p + n) & 31. rs holds 2 x 32
    doubles (alternate steps use alternate halves). False when a pivot's
    magnitude is not above `floor`. */
+template <class G>
 __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor, double *rs,
-                        const Grp &g)
+                        const G &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
+    bool ok = true;
 
     for (int k = 0; k < n; k++) {
         double *r = rs + 32 * (k & 1);
@@ -668,8 +697,8 @@ __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor,
         gsync(g);
         const double d = r[0];
 
-        if (!(fabs(d) > floor))
-            return false;
+        /* a half that met a small pivot stays in step; its values are unused */
+        ok = ok && fabs(d) > floor;
         const double id = rcp_newton(d);
         const bool piv0 = i0 == k, piv1 = i1 == k;
         /* the pivot row scales by 1 / a_kk: a_kj - (1 - 1 / a_kk) a_kj, with
@@ -690,7 +719,7 @@ __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor,
         g0[31] = piv0 ? -id : f0;
         g1[31] = piv1 ? -id : f1;
     }
-    return true;
+    return ok;
 }
 
 /* Rows i0, i1 of a matrix whose register column p is true column
@@ -834,7 +863,7 @@ __device__ __forceinline__ int sym_idx(int n, int i, int j)
 
 /* |T| in double into w.G (packed upper triangle), from T (n <= 32); lane l
    takes rows l and n - 1 - l, so that every lane has n + 1 entries. */
-__device__ void packed_abs_t(int n, int ld, const HWs &w, const Grp &g)
+__device__ void packed_abs_t(int n, int ld, const HWs &w, const Pair &g)
 {
 #pragma unroll
     for (int t = 0; t < 2; t++) {
@@ -865,21 +894,31 @@ __device__ void full_abs_t(double *A, int n, int ld, const double *Gp, const Grp
 /* |T|^-1 into w.G; inv_max receives n max|inv_ij| (infinite when a
    fallback tier ran). */
 __device__ unsigned emi_inverse(int n, int ld, const HWs &w, double *A, double *V, double *lam,
-                                const Grp &g, double &inv_max)
+                                const Pair &pg, double &inv_max)
 {
+    const Grp g = alone(pg);
     const int i0 = g.gl, i1 = g.gl + 16;
     double g0[32], g1[32];
     unsigned st = 0;
     int rot = n;
     bool full = false;
 
-    packed_abs_t(n, ld, w, g);
+    packed_abs_t(n, ld, w, pg);
 #pragma unroll
     for (int j = 0; j < 32; j++) {
         g0[j] = (i0 < n && j < n) ? w.G[sym_idx(n, i0, j)] : 0.0;
         g1[j] = (i1 < n && j < n) ? w.G[sym_idx(n, i1, j)] : 0.0;
     }
-    bool ok = sweep16(g0, g1, n, 1.0e-5, w.rs, g);
+    auto largest = [&]() {
+        double mx = 0.0;
+
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            mx = fmax(mx, fmax(fabs(g0[j]), fabs(g1[j])));
+        return mx;
+    };
+    bool ok = sweep16(g0, g1, n, 1.0e-5, w.rs, pg);
+    double mx = gmaxd(largest(), pg);
 
     if (!ok) {
         /* a pivot of |T| is close to zero: (|T|^2)^-1 |T|, with the
@@ -895,23 +934,14 @@ __device__ unsigned emi_inverse(int n, int ld, const HWs &w, double *A, double *
             gsync(g);
             rows_times(V, A, ld, n, i0, i1, g0, g1);
             rot = 0;
+            mx = gmaxd(largest(), g);
         }
     }
-    if (ok) {
-        /* every |eigenvalue| of |T| above 1e-9, where the pseudo-inverse of
-           reference.py is the inverse: n max|inv_ij| < 1e8 ensures it. */
-        double mx = 0.0;
-
-#pragma unroll
-        for (int j = 0; j < 32; j++)
-            mx = fmax(mx, fmax(fabs(g0[j]), fabs(g1[j])));
-        mx = gmaxd(mx, g);
-        ok = mx == mx && n * mx < 1.0e8;
-        inv_max = ok && !full ? n * mx : INFINITY;
-    }
-    else
-        inv_max = INFINITY;
-    gsync(g);
+    /* every |eigenvalue| of |T| above 1e-9, where the pseudo-inverse of
+       reference.py is the inverse: n max|inv_ij| < 1e8 ensures it. */
+    ok = ok && mx == mx && n * mx < 1.0e8;
+    inv_max = ok && !full ? n * mx : INFINITY;
+    gsync(pg);
     if (ok) {
         const double sc = rot ? -1.0 : 1.0;
 
@@ -935,7 +965,7 @@ __device__ unsigned emi_inverse(int n, int ld, const HWs &w, double *A, double *
             for (int j = r; j < n; j++)
                 w.G[tc_pidx(n, r, j)] = A[r * ld + j];
     }
-    gsync(g);
+    gsync(pg);
     return st;
 }
 
@@ -955,7 +985,8 @@ __device__ __forceinline__ double2 mval(const HWs &w, int ld, int i, int j)
    mapped by Q^H, its component along y removed, the real and imaginary
    parts solved with the LU, the y component removed again, and the result
    mapped back by Q. Scratch: the first 32 float2 of w.x. */
-__device__ void solve_off(int n, int ld, const HWs &w, const Grp &g, const float (&yr)[32],
+template <class G>
+__device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (&yr)[32],
                           unsigned long long piv, float2 b0, float2 b1, float2 &t0, float2 &t1)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
@@ -1001,8 +1032,8 @@ __device__ void solve_off(int n, int ld, const HWs &w, const Grp &g, const float
         tri_solve(v, n, piv, w);
 #pragma unroll
         for (int k = 0; k < 32; k++) {
-            tr_[k] = __shfl_sync(g.mask, v[k], g.base);
-            ti_[k] = __shfl_sync(g.mask, v[k], g.base | 8);
+            tr_[k] = __shfl_sync(g.members(), v[k], g.base);
+            ti_[k] = __shfl_sync(g.members(), v[k], g.base | 8);
         }
     }
     float dr = 0.f, di = 0.f;
@@ -1110,7 +1141,7 @@ template <int B>
 __device__ __forceinline__ void load_T_batch(const float2 (&gv)[B], int t0, int n, int npu, bool active,
                                              int looks, const TcLinkConst &k,
                                              const unsigned short *upper_tab, const HWs &w,
-                                             int ld, const Grp &g, bool &boundary)
+                                             int ld, const Pair &g, bool &boundary)
 {
     const float fl = (float)looks;
     const bool debias = k.bias && looks > 1;
@@ -1168,7 +1199,7 @@ struct TFirst {
 };
 
 __device__ __forceinline__ void t_first(TFirst &f, int n, int p, bool inrange,
-                                        const float2 *__restrict__ gram, const Grp &g)
+                                        const float2 *__restrict__ gram, const Pair &g)
 {
     const int npu = tc_npu(n), i0 = g.gl, i1 = g.gl + 16;
 
@@ -1190,7 +1221,7 @@ __device__ __forceinline__ void t_first(TFirst &f, int n, int p, bool inrange,
    table. */
 __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k, int p, bool active,
                        int looks, const float2 *__restrict__ gram, const TFirst &f,
-                       const unsigned short *upper_tab, const HWs &w, int ld, const Grp &g,
+                       const unsigned short *upper_tab, const HWs &w, int ld, const Pair &g,
                        bool &boundary)
 {
     const int n = s.n, npu = tc_npu(n);
@@ -1212,11 +1243,11 @@ __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
     }
     load_T_batch<16>(gb, 17, n, npu, active, looks, k, upper_tab, w, ld, g, boundary);
     gsync(g);
-    boundary = __any_sync(g.mask, boundary);
+    boundary = ((__ballot_sync(FULL, boundary) >> g.base) & 0xFFFFu) != 0u;
 }
 
 /* Whether the non-zero coherences link all dates (n <= 32). */
-__device__ bool linked16(int n, int ld, const float2 *T, const Grp &g)
+__device__ bool linked16(int n, int ld, const float2 *T, const Pair &g)
 {
     unsigned adj[2] = {0u, 0u};
 
@@ -1244,10 +1275,10 @@ __device__ bool linked16(int n, int ld, const float2 *T, const Grp &g)
             mine |= adj[1];
 #pragma unroll
         for (int o = 8; o; o >>= 1)
-            mine |= __shfl_xor_sync(g.mask, mine, o);
+            mine |= __shfl_xor_sync(g.members(), mine, o);
         const unsigned nw = mine & ~reached;
 
-        if (!nw)
+        if (!__any_sync(FULL, nw != 0u))
             break;
         reached |= nw;
         frontier = nw;
@@ -1258,7 +1289,7 @@ __device__ bool linked16(int n, int ld, const float2 *T, const Grp &g)
 /* Unit phasors relative to the median date (tcoh.cl:700-724) into w.zs,
    then the goodness of fit (tcoh.cl:728-744), pairs spread evenly over the
    lanes. */
-__device__ float gamma16(int n, int ld, const HWs &w, const Grp &g, double2 z0d, double2 z1d,
+__device__ float gamma16(int n, int ld, const HWs &w, const Pair &g, double2 z0d, double2 z1d,
                          const unsigned short *__restrict__ upper_tab, float2 *sum = nullptr)
 {
     /* the phasors in float, as the reference kernel forms them: the
@@ -1271,7 +1302,7 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Grp &g, double2 z0d,
     int ref = n / 2;
     const float mref = gbcast(ref < 16 ? m0 : m1, ref, g);
 
-    if (mref <= 1.0e-3f * mx) {
+    if (__any_sync(FULL, mref <= 1.0e-3f * mx)) {
         int last = -1;
 
         if (i0 < n && m0 == mx)
@@ -1280,8 +1311,9 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Grp &g, double2 z0d,
             last = i1;
 #pragma unroll
         for (int o = 8; o; o >>= 1)
-            last = max(last, __shfl_xor_sync(g.mask, last, o));
-        ref = last;
+            last = max(last, __shfl_xor_sync(g.members(), last, o));
+        if (mref <= 1.0e-3f * mx)
+            ref = last;
     }
     const float zrx = gbcast(ref < 16 ? z0.x : z1.x, ref, g);
     const float zry = gbcast(ref < 16 ? z0.y : z1.y, ref, g);
@@ -1377,7 +1409,7 @@ __device__ __forceinline__ float2 t_full(const HWs &w, int ld, int i, int j)
    owner of row i forms G_ij = (T-bar_ij + conj(T-bar_ji)) / 2 for j > i.
    Db: n x ld double scratch (EMI). An inactive pixel gets G = 0. */
 template <bool EMI>
-__device__ void backward16(int n, int ld, const HWs &w, const Grp &g, double2 z0d, double2 z1d,
+__device__ void backward16(int n, int ld, const HWs &w, const Pair &g, double2 z0d, double2 z1d,
                            float2 S, const float (&yr)[32], unsigned long long piv, int looks,
                            bool bias, bool active, double *Db, float2 *gbar, long long npix,
                            long long p)
@@ -1393,7 +1425,7 @@ __device__ void backward16(int n, int ld, const HWs &w, const Grp &g, double2 z0
     int ref = n / 2;
     const float mref = gbcast(ref < 16 ? mf0 : mf1, ref, g);
 
-    if (mref <= 1.0e-3f * mxf) {
+    if (__any_sync(FULL, mref <= 1.0e-3f * mxf)) {
         int last = -1;
 
         if (i0 < n && mf0 == mxf)
@@ -1402,8 +1434,9 @@ __device__ void backward16(int n, int ld, const HWs &w, const Grp &g, double2 z0
             last = i1;
 #pragma unroll
         for (int o = 8; o; o >>= 1)
-            last = max(last, __shfl_xor_sync(g.mask, last, o));
-        ref = last;
+            last = max(last, __shfl_xor_sync(g.members(), last, o));
+        if (mref <= 1.0e-3f * mxf)
+            ref = last;
     }
     const bool big0 = i0 < n && mf0 > mxf * 1.0e-3f, big1 = i1 < n && mf1 > mxf * 1.0e-3f;
     const double nn = gsum(m0 * m0 + m1 * m1, g);
@@ -1693,7 +1726,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
-    const Grp g = make_grp(lane);
+    const Pair g = make_pair(lane);
     const int grp = warp * 2 + (lane >> 4);
     const HWs w = hws(smem + (size_t)grp * L.per_group, L);
     const int n = s.n, ld = L.ld;
@@ -1773,7 +1806,9 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
 
                     pairs[t * plane + out] = hypotf(tv.x, tv.y);
                 }
-            if (k.bias && active && !linked16(n, ld, w.T, g)) {
+            const bool split = k.bias && !linked16(n, ld, w.T, g);
+
+            if (active && split) {
                 if (g.gl == 0)
                     coh[out] = NAN;
                 if (phases)
@@ -1789,8 +1824,8 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                 for (int r = g.gl; r < n; r += 16)
                     for (int j = 0; j < n; j++)
                         w.T[r * ld + j] = make_float2(r == j ? 1.f : 0.f, 0.f);
-                gsync(g);
             }
+            gsync(g);
             run = __any_sync(FULL, active);
         }
         __syncthreads();
@@ -1870,7 +1905,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                    workload unchanged (3.4e-5) at 6 % less link time. */
                 if (active && sturm16(w.d, w.e2f, n, lambda + TC_REFINE_GAP * norm,
                                       1.0e-30f + 1.0e-14f * norm) >= 2)
-                    refine(n, ld, w, g, z0, z1, yr, piv);
+                    refine(n, ld, w, alone(g), z0, z1, yr, piv);
                 /* Pixels whose gamma the float rounding of T may move by
                    more than ~1e-5 go to the exact tier: the first-order
                    sensitivity of M's eigenvector to T grows with
