@@ -414,9 +414,46 @@ __device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, f
                                    v1[m].y * v1[j].x;
                 }
         }
+        /* Sums over the group by recursive halving, the tree of gsum (lanes
+           8, 4, 2, 1 apart) with each lane keeping half of its values at
+           every level: 15 shuffles for r[0..15], whose total number gl ends
+           in lane gl, and 5 for r[16..19], instead of 80; the totals are
+           then shared through memory. */
+        float *red = (float *)w.x + 128 + 32 * ((b >> 2) & 1);
+
 #pragma unroll
-        for (int e = 0; e < 20; e++)
-            r[e] = gsum(r[e], g);
+        for (int o = 8; o; o >>= 1) {
+            const bool up = (g.gl & o) != 0;
+
+#pragma unroll
+            for (int e = 0; e < o; e++) {
+                const float give = up ? r[e] : r[e + o], keep = up ? r[e + o] : r[e];
+
+                r[e] = keep + __shfl_xor_sync(g.members(), give, o);
+            }
+            if (o >= 4)
+#pragma unroll
+                for (int e = 16; e < 16 + o / 4; e++) {
+                    const float give = up ? r[e] : r[e + o / 4], keep = up ? r[e + o / 4] : r[e];
+
+                    r[e] = keep + __shfl_xor_sync(g.members(), give, o);
+                }
+            else
+                r[16] += __shfl_xor_sync(g.members(), r[16], o);
+        }
+        red[g.gl] = r[0];
+        if ((g.gl & 3) == 0)
+            red[16 + (g.gl >> 2)] = r[16];
+        gsync(g);
+#pragma unroll
+        for (int e = 0; e < 20; e += 4) {
+            const float4 v = *(const float4 *)(red + e);
+
+            r[e] = v.x;
+            r[e + 1] = v.y;
+            r[e + 2] = v.z;
+            r[e + 3] = v.w;
+        }
         float2 h[4];
 
         {
@@ -447,16 +484,31 @@ __device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, f
 }
 
 
+/* The hardware's approximate reciprocal, within two ulps; operands and results
+   are never denormal where it is used. */
+__device__ __forceinline__ float rcp_approx(float x)
+{
+    float y;
+
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+/* Eigenvalues of the group's tridiagonal below x. The chain from one pivot to
+   the next is a reciprocal, a select and a fused multiply-add: the test for a
+   small pivot runs beside the reciprocal. */
 __device__ __forceinline__ int sturm16(const float *d, const float *e2, int n, float x,
                                        float pivmin)
 {
+    const float rsmall = rcp_approx(-pivmin);
     float q = d[0] - x;
     int c = q < 0.f;
 
+#pragma unroll 4
     for (int i = 1; i < n; i++) {
-        if (fabsf(q) < pivmin)
-            q = -pivmin;
-        q = d[i] - x - __fdividef(e2[i - 1], q);
+        const float r = rcp_approx(q);
+
+        q = fmaf(-e2[i - 1], fabsf(q) < pivmin ? rsmall : r, d[i] - x);
         c += q < 0.f;
     }
     return c;
@@ -524,49 +576,65 @@ __device__ float tri_eigenvalue(int n, int index, const HWs &w, const Pair &g, f
     return 0.5f * (lo + hi);
 }
 
-/* The LU's reciprocals (pivots of a shifted tridiagonal) need no correct
-   rounding: the hardware approximation, within two ulps. */
-__device__ __forceinline__ float rcpx(float x) { return __fdividef(1.0f, x); }
+/* Partially pivoted LU of tri - lambda I. Every lane of the group holds it in
+   registers, and the solves of the inverse iteration run on these; the first
+   lane also writes it to w.lu for the solves off the eigenvector. Rows n and
+   up are those of the identity. Straight-line code: the two pixels of a warp
+   pivot differently, and what depends on the pivot is selected (one reciprocal
+   a row). With the factors in shared memory, a branch a row and the pivots'
+   branches taken in turn, the LU and the three solves took 5.0k and 10.0k of
+   the 48k cycles of the eigenvector stage (16 pixels at 30 dates), mostly
+   waiting. This stage as a whole, with the sums of apply_q halved recursively
+   and the shorter chain of sturm16: link stage 94.4 -> 85.7 ms per 512 x 4096
+   AD / EMI / -b strip at 30 dates. */
+struct TriLU {
+    float rd[32], u1[32], u2[32], l[32]; /* 1 / u_kk, u_k,k+1, u_k,k+2, l_k+1,k */
+    unsigned piv;
+};
 
-/* Partially pivoted LU of tri - lambda I, into w.lu (written by the first
-   lane of the group); returns the pivot bits. Every lane computes it. */
-template <typename R>
-__device__ unsigned long long tri_lu(int n, R lambda, R tiny, const HWs &w, const Pair &g)
+__device__ __forceinline__ void tri_lu(TriLU &f, int n, float lambda, float tiny, const HWs &w,
+                                       const Pair &g)
 {
-    R dd = (R)w.d[0] - lambda, s1 = n > 1 ? (R)w.e[0] : (R)0;
-    unsigned long long piv = 0ull;
+    float d[32], e[32];
 
-    for (int k = 0; k < n - 1; k++) {
-        const R sub = w.e[k], nd = (R)w.d[k + 1] - lambda;
-        const R ns = k + 1 < n - 1 ? (R)w.e[k + 1] : (R)0;
-        float4 f;
+#pragma unroll
+    for (int k = 0; k < 32; k += 4) {
+        const float4 a = *(const float4 *)(w.d + k), b = *(const float4 *)(w.e + k);
 
-        if (fabs(dd) >= fabs(sub)) {
-            if (fabs(dd) < tiny)
-                dd = dd < (R)0 ? -tiny : tiny;
-            const R rd = rcpx(dd), l = sub * rd;
-
-            f = make_float4((float)rd, (float)s1, 0.f, (float)l);
-            dd = nd - l * s1;
-            s1 = ns;
-        }
-        else {
-            const R rs = rcpx(sub), l = dd * rs;
-
-            piv |= 1ull << k;
-            f = make_float4((float)rs, (float)nd, (float)ns, (float)l);
-            dd = s1 - l * nd;
-            s1 = -l * ns;
-        }
-        if (g.gl == 0)
-            w.lu[k] = f;
+        d[k] = k < n ? a.x : 0.f;
+        d[k + 1] = k + 1 < n ? a.y : 0.f;
+        d[k + 2] = k + 2 < n ? a.z : 0.f;
+        d[k + 3] = k + 3 < n ? a.w : 0.f;
+        e[k] = k < n - 1 ? b.x : 0.f;
+        e[k + 1] = k + 1 < n - 1 ? b.y : 0.f;
+        e[k + 2] = k + 2 < n - 1 ? b.z : 0.f;
+        e[k + 3] = k + 3 < n - 1 ? b.w : 0.f;
     }
-    if (fabs(dd) < tiny)
-        dd = dd < (R)0 ? -tiny : tiny;
-    if (g.gl == 0)
-        w.lu[n - 1] = make_float4((float)rcpx(dd), 0.f, 0.f, 0.f);
+    float dd = d[0] - lambda, s1 = e[0];
+
+    f.piv = 0u;
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+        const float sub = e[k], nd = k < 31 ? d[k + 1] - lambda : 0.f;
+        const float ns = k < 31 ? e[k + 1] : 0.f;
+        const bool swap = !(fabsf(dd) >= fabsf(sub));
+        const float dc = fabsf(dd) < tiny ? (dd < 0.f ? -tiny : tiny) : dd;
+        const float r = rcp_approx(swap ? sub : dc);
+        const float l = (swap ? dd : sub) * r;
+        const float m = swap ? nd : s1, o = swap ? s1 : nd;
+
+        f.rd[k] = k < n ? r : 1.f;
+        f.u1[k] = m;
+        f.u2[k] = swap ? ns : 0.f;
+        f.l[k] = l;
+        if (swap)
+            f.piv |= 1u << k;
+        if (g.gl == 0)
+            w.lu[k] = make_float4(r, m, f.u2[k], l);
+        dd = fmaf(-l, m, o);
+        s1 = swap ? -l * ns : ns;
+    }
     gsync(g);
-    return piv;
 }
 
 /* Solve (tri - lambda) with the LU of tri_lu, in place on yr (every lane,
@@ -601,6 +669,28 @@ __device__ __forceinline__ void tri_solve(float (&yr)[32], int n, unsigned long 
     }
 }
 
+__device__ __forceinline__ void tri_solve(float (&yr)[32], const TriLU &f)
+{
+#pragma unroll
+    for (int k = 0; k < 31; k++) {
+        const bool swap = ((f.piv >> k) & 1u) != 0u;
+        const float a = swap ? yr[k + 1] : yr[k], b = swap ? yr[k] : yr[k + 1];
+
+        yr[k] = a;
+        yr[k + 1] = fmaf(-f.l[k], a, b);
+    }
+#pragma unroll
+    for (int k = 31; k >= 0; k--) {
+        float v = yr[k];
+
+        if (k < 31)
+            v = fmaf(-f.u1[k], yr[k + 1], v);
+        if (k < 30)
+            v = fmaf(-f.u2[k], yr[k + 2], v);
+        yr[k] = v * f.rd[k];
+    }
+}
+
 /* The eigenvector of rank `index` of the reduced matrix, back-transformed:
    returns the components of rows i0, i1 in z0, z1; y (tridiagonal vector)
    is left in yr. */
@@ -613,19 +703,23 @@ __device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g
     lambda = tri_eigenvalue(n, index, w, g, norm, status);
     const float tiny = 1.0e-6f * fmaxf(norm, 1.0e-30f);
 
-    piv = tri_lu<float>(n, lambda, tiny, w, g);
+    TriLU f;
 
+    tri_lu(f, n, lambda, tiny, w, g);
+    piv = f.piv;
 #pragma unroll
     for (int k = 0; k < 32; k++)
         yr[k] = 1.f;
     for (int it = 0; it < 3; it++) {
-        tri_solve(yr, n, piv, w);
-        float nrm = 0.f;
+        tri_solve(yr, f);
+        float nrm = 0.f, odd = 0.f;
 
 #pragma unroll
-        for (int k = 0; k < 32; k++)
-            if (k < n)
-                nrm = fmaxf(nrm, fabsf(yr[k]));
+        for (int k = 0; k < 32; k += 2) {
+            nrm = fmaxf(nrm, k < n ? fabsf(yr[k]) : 0.f);
+            odd = fmaxf(odd, k + 1 < n ? fabsf(yr[k + 1]) : 0.f);
+        }
+        nrm = fmaxf(nrm, odd);
         const float inv = __frcp_rn(nrm);
 
 #pragma unroll
@@ -1246,42 +1340,25 @@ __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
     boundary = ((__ballot_sync(FULL, boundary) >> g.base) & 0xFFFFu) != 0u;
 }
 
-/* Whether the non-zero coherences link all dates (n <= 32). */
+/* Whether the non-zero coherences link all dates (n <= 32): the dates
+   reached from date 0, expanded one at a time (a vote over the lanes' entries
+   of its row; most often one or two rows reach every date). */
 __device__ bool linked16(int n, int ld, const float2 *T, const Pair &g)
 {
-    unsigned adj[2] = {0u, 0u};
-
-#pragma unroll
-    for (int t = 0; t < 2; t++) {
-        const int r = g.gl + 16 * t;
-
-        if (r < n)
-            for (int j = 0; j < n; j++) {
-                const float2 v = T[r * ld + j];
-
-                if (j != r && (v.x != 0.f || v.y != 0.f))
-                    adj[t] |= 1u << j;
-            }
-    }
+    const int i0 = g.gl, i1 = g.gl + 16;
     const unsigned all = n == 32 ? ~0u : (1u << n) - 1u;
-    unsigned reached = 1u, frontier = 1u;
+    unsigned reached = 1u, todo = 1u;
 
-    for (int it = 0; it < n; it++) {
-        unsigned mine = 0u;
+    while (__any_sync(FULL, todo != 0u && reached != all)) {
+        const int f = todo ? __ffs(todo) - 1 : 0;
+        const float2 a = i0 < n ? T[f * ld + i0] : make_float2(0.f, 0.f);
+        const float2 b = i1 < n ? T[f * ld + i1] : make_float2(0.f, 0.f);
+        const unsigned lo = __ballot_sync(FULL, a.x != 0.f || a.y != 0.f) >> g.base;
+        const unsigned hi = __ballot_sync(FULL, b.x != 0.f || b.y != 0.f) >> g.base;
+        const unsigned nw = ((lo & 0xFFFFu) | (hi << 16)) & ~reached;
 
-        if ((frontier >> g.gl) & 1u)
-            mine |= adj[0];
-        if (g.gl + 16 < n && ((frontier >> (g.gl + 16)) & 1u))
-            mine |= adj[1];
-#pragma unroll
-        for (int o = 8; o; o >>= 1)
-            mine |= __shfl_xor_sync(g.members(), mine, o);
-        const unsigned nw = mine & ~reached;
-
-        if (!__any_sync(FULL, nw != 0u))
-            break;
         reached |= nw;
-        frontier = nw;
+        todo = (todo & (todo - 1u)) | nw;
     }
     return reached == all;
 }
