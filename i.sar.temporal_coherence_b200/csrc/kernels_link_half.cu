@@ -48,6 +48,8 @@
 
 namespace {
 
+constexpr int LT_BATCH = 6; /* entries of T per lane and turn of load_T */
+
 /* A half-warp. Collectives take their mask from members(): Pair, for code
    that both halves of the warp run together, names all 32 lanes, a constant
    (shuffles, votes and warp barriers with a mask that is only known at run
@@ -115,6 +117,15 @@ __device__ __forceinline__ float gminf(float v, const G &g)
 }
 
 template <class G>
+__device__ __forceinline__ unsigned gmaxu(unsigned v, const G &g)
+{
+#pragma unroll
+    for (int o = 8; o; o >>= 1)
+        v = max(v, __shfl_xor_sync(g.members(), v, o));
+    return v;
+}
+
+template <class G>
 __device__ __forceinline__ double gmaxd(double v, const G &g)
 {
 #pragma unroll
@@ -138,8 +149,8 @@ __device__ __forceinline__ void gsync(const G &g)
 /* Per-group shared workspace (byte offsets, 16-byte aligned). */
 struct HalfLayout {
     int n, ld;
-    int off_T, off_G, off_vw, off_lu, off_tau, off_d, off_e, off_df, off_e2f, off_y,
-        off_nrm, off_zs, off_rs, off_lam, off_x, off_Db;
+    int off_T, off_G, off_vw, off_lu, off_tau, off_d, off_e, off_e2f, off_nrm, off_zs, off_rs,
+        off_x, off_Db;
     int per_group;
 };
 
@@ -150,9 +161,10 @@ struct HWs {
     float4 *vw;
     float4 *lu;
     float2 *tau;
-    float *d, *e, *df, *e2f, *y, *nrm; /* nrm: 1 / sqrt(C_ii) */
+    float *y;       /* the tridiagonal eigenvector, for refine */
+    float *d, *e, *e2f, *nrm; /* nrm: 1 / sqrt(C_ii) */
     float2 *zs;
-    double *rs, *lam;
+    double *rs;
     double2 *x; /* scratch vectors of the adjoint's solves (2 x 32) */
 };
 
@@ -168,14 +180,12 @@ __device__ __forceinline__ HWs hws(unsigned char *base, const HalfLayout &L)
     w.tau = (float2 *)(base + L.off_tau);
     w.d = (float *)(base + L.off_d);
     w.e = (float *)(base + L.off_e);
-    w.df = (float *)(base + L.off_df);
     w.e2f = (float *)(base + L.off_e2f);
-    w.y = (float *)(base + L.off_y);
     w.nrm = (float *)(base + L.off_nrm);
     w.zs = (float2 *)(base + L.off_zs);
     w.rs = (double *)(base + L.off_rs);
-    w.lam = nullptr;
     w.x = (double2 *)(base + L.off_x);
+    w.y = (float *)(base + L.off_x) + 192; /* beyond x and apply_q's sums */
     return w;
 }
 
@@ -494,6 +504,15 @@ __device__ __forceinline__ float rcp_approx(float x)
     return y;
 }
 
+/* The approximate reciprocal square root, likewise. */
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float y;
+
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 /* Eigenvalues of the group's tridiagonal below x. The chain from one pivot to
    the next is a reciprocal, a select and a fused multiply-add: the test for a
    small pivot runs beside the reciprocal. */
@@ -772,46 +791,56 @@ __device__ __forceinline__ double rcp_newton(double d)
    symmetric, pivot row k is assembled from every lane's own column-k
    entries. The register columns rotate by one per step so that the pivot
    column is always g[0] (the step loop stays a run-time loop): on return
-   register column p holds true column (p + n) & 31. rs holds 2 x 32
-   doubles (alternate steps use alternate halves). False when a pivot's
-   magnitude is not above `floor`. */
+   register column p holds true column (p + n) & 31. Each step updates the
+   next pivot column first and publishes it, so that the next pivot's
+   reciprocal (a chain of eight dependent operations) forms while the other
+   columns update. rs holds 3 x 32 doubles, taken in turn: a step writes the
+   buffer that was last read before the barrier of the step before it. False
+   when a pivot's magnitude is not above `floor`. */
 template <class G>
 __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor, double *rs,
                         const G &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
-    bool ok = true;
+    /* a_ik, in the order of the registers: r[p] = a_k,(p + k) & 31 */
+    double *r = rs;
+
+    r[i0] = g0[0];
+    r[i1] = g1[0];
+    gsync(g);
+    /* a half that met a small pivot stays in step; its values are unused */
+    bool ok = fabs(r[0]) > floor;
+    double id = rcp_newton(r[0]);
 
     for (int k = 0; k < n; k++) {
-        double *r = rs + 32 * (k & 1);
-
-        /* a_ik, in the order of the registers: rs[p] = a_k,(p + k) & 31 */
-        r[(i0 - k) & 31] = g0[0];
-        r[(i1 - k) & 31] = g1[0];
-        gsync(g);
-        const double d = r[0];
-
-        /* a half that met a small pivot stays in step; its values are unused */
-        ok = ok && fabs(d) > floor;
-        const double id = rcp_newton(d);
         const bool piv0 = i0 == k, piv1 = i1 == k;
         /* the pivot row scales by 1 / a_kk: a_kj - (1 - 1 / a_kk) a_kj, with
            a_kj from rs (equal to the row's own value up to rounding) */
         const double f0 = piv0 ? 1.0 - id : g0[0] * id, f1 = piv1 ? 1.0 - id : g1[0] * id;
+        double *rn = r == rs + 64 ? rs : r + 32;
+        const double a1 = r[1];
+
+        g0[0] = fma(-f0, a1, g0[1]);
+        g1[0] = fma(-f1, a1, g1[1]);
+        rn[(i0 - k - 1) & 31] = g0[0];
+        rn[(i1 - k - 1) & 31] = g1[0];
+        gsync(g);
+        const double dn = rn[0], idn = rcp_newton(dn); /* unused after the last step */
 
 #pragma unroll
-        for (int q = 0; q < 32; q += 2) {
+        for (int q = 2; q < 32; q += 2) {
             const double2 a = *(const double2 *)&r[q];
 
-            if (q > 0) {
-                g0[q - 1] = fma(-f0, a.x, g0[q]);
-                g1[q - 1] = fma(-f1, a.x, g1[q]);
-            }
+            g0[q - 1] = fma(-f0, a.x, g0[q]);
+            g1[q - 1] = fma(-f1, a.x, g1[q]);
             g0[q] = fma(-f0, a.y, g0[q + 1]);
             g1[q] = fma(-f1, a.y, g1[q + 1]);
         }
         g0[31] = piv0 ? -id : f0;
         g1[31] = piv1 ? -id : f1;
+        r = rn;
+        id = idn;
+        ok = ok && (k == n - 1 || fabs(dn) > floor);
     }
     return ok;
 }
@@ -955,109 +984,223 @@ __device__ __forceinline__ int sym_idx(int n, int i, int j)
     return i <= j ? tc_pidx(n, i, j) : tc_pidx(n, j, i);
 }
 
-/* |T| in double into w.G (packed upper triangle), from T (n <= 32); lane l
-   takes rows l and n - 1 - l, so that every lane has n + 1 entries. */
-__device__ void packed_abs_t(int n, int ld, const HWs &w, const Pair &g)
+/* |t| in double: the squares of the float parts are exact, their sum is
+   rounded once; the root by two Newton steps (s += (m - s^2) / (2 s), in the
+   form s += e h with h = 1 / (2 s) from the float reciprocal root, relative
+   error 2^-22 -> 2^-43 -> rounding), 0 below 3e-19. The library's root and
+   hypot branch, which keeps the entries of a batch from overlapping. ADJ:
+   hypot, within an ulp of it (the gradients of nearly degenerate pixels
+   magnify even that). */
+template <bool ADJ>
+__device__ __forceinline__ double abs_t(float2 t)
 {
-#pragma unroll
-    for (int t = 0; t < 2; t++) {
-        const int r = t ? n - 1 - g.gl : g.gl;
+    const double x = t.x, y = t.y;
 
-        if (r < n && (t == 0 ? r <= n - 1 - g.gl : r > g.gl))
-            for (int j = r; j < n; j++) {
-                const float2 v = w.T[r * ld + j];
+    if (ADJ)
+        return hypot(x, y);
+    const double m = fma(x, x, y * y);
+    const float mf = fmaf(t.x, t.x, t.y * t.y);
+    const double y0 = mf > 1.0e-37f ? rsqrt_approx(mf) : 0.f, h = 0.5 * y0;
+    double s = m * y0;
 
-                w.G[tc_pidx(n, r, j)] = hypot((double)v.x, (double)v.y);
-            }
-    }
-    gsync(g);
+    s = fma(fma(-s, s, m), h, s);
+    return fma(fma(-s, s, m), h, s);
 }
 
-/* |T| in full into A (n x ld, global scratch), from its packed copy. */
-__device__ void full_abs_t(double *A, int n, int ld, const double *Gp, const Grp &g)
+/* The slot of a lower-triangle entry of T, which the link stages use in turn
+   for |T_ij| (double), M_ij and the Householder vectors (float2). */
+__device__ __forceinline__ double &abs_slot(const HWs &w, int ld, int i, int j)
 {
+    return *(double *)&w.T[i * ld + j];
+}
+
+/* The rare fallback tiers of |T|^-1, into A (n x ld, global scratch; V, n x
+   ld, and lam, n: workspaces): through |T|^2 when a pivot of |T| is close to
+   zero (`squared`), by the Jacobi pseudo-inverse when that fails too or the
+   inverse is too large. */
+template <bool ADJ>
+__device__ __noinline__ unsigned emi_fallback(int n, int ld, HWs w, double *A, double *V,
+                                              double *lam, Grp g, bool squared)
+{
+    const int i0 = g.gl, i1 = g.gl + 16;
+
     for (int r = g.gl; r < n; r += 16)
         for (int j = 0; j < n; j++)
-            A[r * ld + j] = Gp[sym_idx(n, r, j)];
+            A[r * ld + j] = r == j ? 1.0 : abs_t<ADJ>(w.T[min(r, j) * ld + max(r, j)]);
     gsync(g);
+    if (squared) {
+        /* (|T|^2)^-1 |T|, with the intermediate inverse in V */
+        double g0[32], g1[32];
+
+        rows_times(A, A, ld, n, i0, i1, g0, g1);
+        if (sweep16(g0, g1, n, 1.0e-300, w.rs, g)) {
+            double mx = 0.0;
+
+            store_rows(V, ld, n, n, -1.0, g0, g1, g);
+            gsync(g);
+            rows_times(V, A, ld, n, i0, i1, g0, g1);
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                mx = fmax(mx, fmax(fabs(g0[j]), fabs(g1[j])));
+            mx = gmaxd(mx, g);
+            if (mx == mx && n * mx < 1.0e8) {
+                gsync(g);
+                store_rows(A, ld, n, 0, 1.0, g0, g1, g);
+                gsync(g);
+                return TC_STATUS_EMI_PINV;
+            }
+        }
+    }
+    return TC_STATUS_EMI_PINV | jacobi_pinv16(n, ld, A, V, lam, g);
 }
 
-/* |T|^-1 into w.G (packed upper triangle, double), from T. The rare
-   fallback tiers work on full matrices A, V (n x ld each) and lam (n) in
-   the group's global scratch. Returns status bits. */
-/* |T|^-1 into w.G; inv_max receives n max|inv_ij| (infinite when a
-   fallback tier ran). */
-__device__ unsigned emi_inverse(int n, int ld, const HWs &w, double *A, double *V, double *lam,
-                                const Pair &pg, double &inv_max)
+/* Index of entry (i, j) of a Hermitian matrix kept left of the diagonal, for j
+   known at compile time. Rows i0 < 16 are right of the diagonal from column 16
+   on and rows i1 >= 16 left of it up to column 15; only the diagonal blocks
+   select. EMI's T has 32 rows, those from n on zero, so that entries beyond n
+   need no test. */
+/* A value that the compiler cannot follow: the addresses formed from it are
+   not kept in registers from one pixel pair to the next (there are more of
+   them than registers; they would be spilled). */
+__device__ __forceinline__ int opaque(int v)
+{
+    asm volatile("" : "+r"(v));
+    return v;
+}
+
+#define TC_LOWER(i, j) ((i) > (j) ? (i) * ld + (j) : (j) * ld + (i))
+
+/* Rows i0, i1 of |T| from the slots that load_T filled. */
+__device__ __forceinline__ void load_abs(double (&g0)[32], double (&g1)[32], int ld_,
+                                         const HWs &w, const Pair &g)
+{
+    const int i0 = g.gl, i1 = g.gl + 16, ld = opaque(ld_);
+    const double *A = (const double *)w.T;
+
+#pragma unroll
+    for (int j = 0; j < 32; j++) {
+        g0[j] = A[j >= 16 ? j * ld + i0 : TC_LOWER(i0, j)];
+        g1[j] = A[j < 16 ? i1 * ld + j : TC_LOWER(i1, j)];
+    }
+}
+
+/* |T|^-1 into w.G (packed upper triangle, double) and M = |T|^-1 o T rounded
+   to float into T's lower triangle and diagonal (M_ij, i >= j): every lane
+   forms the entries left of the diagonal in its rows from the inverse that it
+   holds, with all column indices static (the register columns are shifted back
+   to the true ones first), without branches. The link stage is bound by the
+   latency of one warp's instructions (two warps per scheduler) and by their
+   fetching, so short straight code with its loads first counts: |T| formed in
+   load_T, this function, the rows of M and load_T as a loop took the link
+   stage from 85.7 to 75.5 ms per 512 x 4096 AD / EMI / -b strip at 30 dates. A, V, lam: the group's global
+   scratch for the rare fallback tiers. inv_max receives n max|inv_ij|
+   (infinite when a fallback tier ran). Returns status bits. */
+template <bool ADJ>
+__device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V, double *lam,
+                               const Pair &pg, double &inv_max)
 {
     const Grp g = alone(pg);
     const int i0 = g.gl, i1 = g.gl + 16;
     double g0[32], g1[32];
     unsigned st = 0;
-    int rot = n;
-    bool full = false;
 
-    packed_abs_t(n, ld, w, pg);
+    load_abs(g0, g1, ld, w, pg);
+    const bool swept = sweep16(g0, g1, n, 1.0e-5, w.rs, pg);
+
+    for (int k = n; k < 32; k++) {
+        const double t0 = g0[0], t1 = g1[0];
+
+#pragma unroll
+        for (int q = 0; q < 31; q++) {
+            g0[q] = g0[q + 1];
+            g1[q] = g1[q + 1];
+        }
+        g0[31] = t0;
+        g1[31] = t1;
+    }
+    /* the largest magnitude left of the diagonal, as an integer: the upper
+       words first, then the lower words of those that have the largest (64
+       double maxima held 64 magnitudes at once and spilled) */
+    unsigned top = 0u, low = 0u;
+
 #pragma unroll
     for (int j = 0; j < 32; j++) {
-        g0[j] = (i0 < n && j < n) ? w.G[sym_idx(n, i0, j)] : 0.0;
-        g1[j] = (i1 < n && j < n) ? w.G[sym_idx(n, i1, j)] : 0.0;
+        if (j < 16)
+            top = max(top, (unsigned)__double2hiint(g0[j]) & 0x7fffffffu);
+        top = max(top, (unsigned)__double2hiint(g1[j]) & 0x7fffffffu);
     }
-    auto largest = [&]() {
-        double mx = 0.0;
-
+    top = gmaxu(top, pg);
 #pragma unroll
-        for (int j = 0; j < 32; j++)
-            mx = fmax(mx, fmax(fabs(g0[j]), fabs(g1[j])));
-        return mx;
-    };
-    bool ok = sweep16(g0, g1, n, 1.0e-5, w.rs, pg);
-    double mx = gmaxd(largest(), pg);
-
-    if (!ok) {
-        /* a pivot of |T| is close to zero: (|T|^2)^-1 |T|, with the
-           intermediate inverse in V */
-        st |= TC_STATUS_EMI_PINV;
-        gsync(g);
-        full_abs_t(A, n, ld, w.G, g);
-        full = true;
-        rows_times(A, A, ld, n, i0, i1, g0, g1);
-        ok = sweep16(g0, g1, n, 1.0e-300, w.rs, g);
-        if (ok) {
-            store_rows(V, ld, n, n, -1.0, g0, g1, g);
-            gsync(g);
-            rows_times(V, A, ld, n, i0, i1, g0, g1);
-            rot = 0;
-            mx = gmaxd(largest(), g);
-        }
+    for (int j = 0; j < 32; j++) {
+        if (j < 16 && ((unsigned)__double2hiint(g0[j]) & 0x7fffffffu) == top)
+            low = max(low, (unsigned)__double2loint(g0[j]));
+        if (((unsigned)__double2hiint(g1[j]) & 0x7fffffffu) == top)
+            low = max(low, (unsigned)__double2loint(g1[j]));
     }
+    const double mx = __hiloint2double((int)top, (int)gmaxu(low, pg));
     /* every |eigenvalue| of |T| above 1e-9, where the pseudo-inverse of
        reference.py is the inverse: n max|inv_ij| < 1e8 ensures it. */
-    ok = ok && mx == mx && n * mx < 1.0e8;
-    inv_max = ok && !full ? n * mx : INFINITY;
-    gsync(pg);
-    if (ok) {
-        const double sc = rot ? -1.0 : 1.0;
+    const bool ok = swept && mx == mx && n * mx < 1.0e8;
+
+    inv_max = ok ? n * mx : INFINITY;
+    {
+        /* rows that store: none of a half that takes a fallback tier */
+        const int e0 = ok && i0 < n ? i0 : -1, e1 = ok && i1 < n ? i1 : -1, lv = opaque(ld);
+
+        /* batches of eight columns: their loads, arithmetic, stores; the
+           diagonal's T is 1 */
+#pragma unroll
+        for (int jb = 0; jb < 32; jb += 8) {
+            float2 m0[8], m1[8];
 
 #pragma unroll
-        for (int p = 0; p < 32; p++) {
-            const int j = (p + rot) & 31;
+            for (int u = 0; u < 8; u++) {
+                if (jb < 16)
+                    m0[u] = w.T[(jb + u) * lv + i0];
+                m1[u] = w.T[(jb + u) * lv + i1];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int j = jb + u;
 
-            if (j < n) {
-                if (i0 <= j)
-                    w.G[tc_pidx(n, i0, j)] = sc * g0[p];
-                if (i1 <= j)
-                    w.G[tc_pidx(n, i1, j)] = sc * g1[p];
+                if (jb < 16) {
+                    if (j == i0)
+                        m0[u] = make_float2(1.f, 0.f);
+                    m0[u] = make_float2((float)(-g0[j] * (double)m0[u].x),
+                                        (float)(g0[j] * (double)m0[u].y));
+                }
+                else if (j == i1)
+                    m1[u] = make_float2(1.f, 0.f);
+                m1[u] = make_float2((float)(-g1[j] * (double)m1[u].x),
+                                    (float)(g1[j] * (double)m1[u].y));
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int j = jb + u;
+                double *gj = w.G + (tc_pidx(n, j, j) - j); /* used where j < n */
+
+                if (jb < 16 && j <= e0) {
+                    w.T[i0 * lv + j] = m0[u];
+                    gj[i0] = -g0[j];
+                }
+                if (j <= e1) {
+                    w.T[i1 * lv + j] = m1[u];
+                    gj[i1] = -g1[j];
+                }
             }
         }
     }
-    else {
-        if (!full)
-            full_abs_t(A, n, ld, w.G, g);
-        st |= TC_STATUS_EMI_PINV | jacobi_pinv16(n, ld, A, V, lam, g);
+    if (!ok) {
+        st |= emi_fallback<ADJ>(n, ld, w, A, V, lam, g, !swept);
         for (int r = g.gl; r < n; r += 16)
-            for (int j = r; j < n; j++)
-                w.G[tc_pidx(n, r, j)] = A[r * ld + j];
+            for (int j = 0; j <= r; j++) {
+                const double a = A[r * ld + j];
+                const float2 t = j == r ? make_float2(1.f, 0.f) : w.T[j * ld + r];
+
+                w.T[r * ld + j] =
+                    make_float2((float)(a * (double)t.x), -(float)(a * (double)t.y));
+                w.G[tc_pidx(n, j, r)] = a;
+            }
     }
     gsync(pg);
     return st;
@@ -1067,7 +1210,7 @@ __device__ unsigned emi_inverse(int n, int ld, const HWs &w, double *A, double *
 __device__ __forceinline__ double2 mval(const HWs &w, int ld, int i, int j)
 {
     const double gg = w.G[sym_idx(w.n, i, j)];
-    const float2 t = w.T[i < j ? i * ld + j : j * ld + i];
+    const float2 t = i == j ? make_float2(1.f, 0.f) : w.T[i < j ? i * ld + j : j * ld + i];
 
     return make_double2(gg * (double)t.x, i < j ? gg * (double)t.y : -gg * (double)t.y);
 }
@@ -1158,9 +1301,10 @@ __device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (
    reduction of M; y is the tridiagonal eigenvector. The residual is formed
    in double; the correction, a small vector that needs only float relative
    accuracy, is mapped through Q in float after scaling the residual to a
-   unit maximum. */
-__device__ void refine(int n, int ld, const HWs &w, const Grp &g, double2 &x0, double2 &x1,
-                       const float (&yr)[32], unsigned long long piv)
+   unit maximum. Few pixels come here: a function of its own, so that its
+   registers are not the common path's. */
+__device__ __noinline__ double4 refine(int n, int ld, HWs w, Grp g, double2 x0, double2 x1,
+                                       unsigned long long piv)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
 
@@ -1211,84 +1355,109 @@ __device__ void refine(int n, int ld, const HWs &w, const Grp &g, double2 &x0, d
 
     gsync(g);
     if (!(rmax > 0.0))
-        return;
+        return make_double4(x0.x, x0.y, x1.x, x1.y);
     const double sc = 1.0 / rmax;
     float2 t0, t1;
+    float yr[32];
+
+#pragma unroll
+    for (int k = 0; k < 32; k++)
+        yr[k] = w.y[k];
 
     solve_off(n, ld, w, g, yr, piv, make_float2((float)(r0.x * sc), (float)(r0.y * sc)),
               make_float2((float)(r1.x * sc), (float)(r1.y * sc)), t0, t1);
-    /* x -= Q (tri - mu)^+ Q^H r */
-    x0.x -= rmax * t0.x;
-    x0.y -= rmax * t0.y;
-    x1.x -= rmax * t1.x;
-    x1.y -= rmax * t1.y;
     gsync(g);
+    /* x -= Q (tri - mu)^+ Q^H r */
+    return make_double4(x0.x - rmax * t0.x, x0.y - rmax * t0.y, x1.x - rmax * t1.x,
+                        x1.y - rmax * t1.y);
 }
 
 /* ------------------------------------------------------------------ */
 /* Common stages.                                                      */
 /* ------------------------------------------------------------------ */
 
-/* One batch of the packed entries q = gl + 16 t (t = t0 .. t0 + B - 1):
-   T_ij = C_ij / (nrm_i nrm_j), bias-corrected, both triangles. */
-template <int B>
-__device__ __forceinline__ void load_T_batch(const float2 (&gv)[B], int t0, int n, int npu, bool active,
-                                             int looks, const TcLinkConst &k,
+/* The packed entries q = gl + 16 (t0 + u), u < LT_BATCH, of the sums gv: T_ij
+   = C_ij / (nrm_i nrm_j), bias-corrected. EVD: both triangles, as its rows are
+   loaded whole; EMI: the upper one, and |T_ij| in double in the lower one's and
+   the diagonal's slots. All loads first, then all arithmetic, then all stores
+   (they are all in shared memory, and the compiler keeps their order), without
+   branches, so that the entries' chains overlap. */
+template <bool EMI, bool ADJ>
+__device__ __forceinline__ void load_T_batch(const float2 (&gv)[LT_BATCH], int t0, int npu,
+                                             bool active, float fl, float ilm1, bool debias,
                                              const unsigned short *upper_tab, const HWs &w,
                                              int ld, const Pair &g, bool &boundary)
 {
-    const float fl = (float)looks;
-    const bool debias = k.bias && looks > 1;
-    const float ilm1 = debias ? __frcp_rn(fl - 1.0f) : 0.f;
+    constexpr int B = LT_BATCH;
+    int ij[B];
+    float rd[B];
+    float2 tv[B];
+    double a[B];
 
 #pragma unroll
-    for (int t = 0; t < B; t++) {
-        const int q = g.gl + 16 * (t0 + t);
+    for (int u = 0; u < B; u++)
+        ij[u] = upper_tab[min(g.gl + 16 * (t0 + u), npu - 1)];
+    /* w.nrm holds 1 / sqrt(C_ii) (0 for an empty date) */
+#pragma unroll
+    for (int u = 0; u < B; u++)
+        rd[u] = w.nrm[ij[u] >> 8] * w.nrm[ij[u] & 255];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+        const float2 gq = gv[u];
+        const bool some = active && rd[u] > 0.f;
 
-        if (q >= npu)
-            continue;
-        const int i = upper_tab[q] >> 8, j = upper_tab[q] & 255;
+        tv[u] = make_float2(some ? gq.x * rd[u] : 0.f, some ? gq.y * rd[u] : 0.f);
+        /* bias correction: f^2 = m2c / m2, m2c = (L m2 - 1) / (L - 1) */
+        const float m2 = fmaf(tv[u].y, tv[u].y, tv[u].x * tv[u].x);
+        const float lm1 = fmaf(fl, m2, -1.0f);
+        const float m2c = lm1 * ilm1;
+        const float f2 = m2c * rcp_approx(m2);
+        const float f = m2 > 0.f && m2c > 0.f && f2 > 0.f ? f2 * rsqrt_approx(f2) : 0.f;
+        const bool edge = fabsf(lm1) < TC_BIAS_BAND * fl * m2;
 
-        if (i == j) {
-            w.T[i * ld + i] = make_float2(1.f, 0.f);
-            continue;
-        }
-        float re = 0.f, im = 0.f;
+        boundary |= debias & edge & ((ij[u] >> 8) != (ij[u] & 255));
+        tv[u].x *= debias ? f : 1.f;
+        tv[u].y *= debias ? f : 1.f;
+        if (EMI)
+            a[u] = abs_t<ADJ>(tv[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+        const int i = ij[u] >> 8, j = ij[u] & 255;
 
-        if (active) {
-            /* w.nrm holds 1 / sqrt(C_ii) (0 for an empty date) */
-            const float2 gq = gv[t];
-            const float rd = w.nrm[i] * w.nrm[j];
-
-            if (rd > 0.f) {
-                re = gq.x * rd;
-                im = gq.y * rd;
-                if (debias) {
-                    /* f^2 = m2c / m2, m2c = (L m2 - 1) / (L - 1) */
-                    const float m2 = re * re + im * im;
-                    const float lm1 = fmaf(fl, m2, -1.0f);
-                    const float m2c = lm1 * ilm1;
-
-                    boundary |= fabsf(lm1) < TC_BIAS_BAND * fl * m2;
-                    const float f2 = m2 > 0.f && m2c > 0.f ? m2c * __fdividef(1.0f, m2) : 0.f;
-                    const float f = f2 > 0.f ? f2 * rsqrtf(f2) : 0.f;
-
-                    re *= f;
-                    im *= f;
-                }
+        if (g.gl + 16 * (t0 + u) < npu) {
+            if (EMI) {
+                if (i != j)
+                    w.T[i * ld + j] = tv[u];
+                abs_slot(w, ld, j, i) = i == j ? 1.0 : a[u];
+            }
+            else {
+                w.T[i * ld + j] = i == j ? make_float2(1.f, 0.f) : tv[u];
+                if (i != j)
+                    w.T[j * ld + i] = make_float2(tv[u].x, -tv[u].y);
             }
         }
-        w.T[i * ld + j] = make_float2(re, im);
-        w.T[j * ld + i] = make_float2(re, -im);
     }
 }
 
-/* The first batch of a pixel's packed Gram sums (entries gl + 16 t, t < 17)
-   and its two diagonal sums, loaded for load_T (zero where out of range).
-   The link kernel issues these loads for the next pixel pair during the
-   last stage of the current one, so that they arrive while gamma runs. */
+/* A batch of a pixel's packed Gram sums (zero where out of range). */
+__device__ __forceinline__ void gram_batch(float2 (&v)[LT_BATCH], int t0, int npu, bool inrange,
+                                           const float2 *__restrict__ sums, const Pair &g)
+{
+#pragma unroll
+    for (int u = 0; u < LT_BATCH; u++) {
+        const int q = g.gl + 16 * (t0 + u);
+
+        v[u] = (inrange && q < npu) ? sums[q] : make_float2(0.f, 0.f);
+    }
+}
+
+/* The first two batches of a pixel's packed Gram sums and its two diagonal
+   sums, loaded for load_T. The link kernel issues these loads for the next
+   pixel pair during the last stage of the current one, so that they arrive
+   while gamma runs. */
 struct TFirst {
-    float2 ga[17];
+    float2 a[LT_BATCH], b[LT_BATCH];
     float d0, d1;
 };
 
@@ -1296,23 +1465,22 @@ __device__ __forceinline__ void t_first(TFirst &f, int n, int p, bool inrange,
                                         const float2 *__restrict__ gram, const Pair &g)
 {
     const int npu = tc_npu(n), i0 = g.gl, i1 = g.gl + 16;
+    const float2 *sums = gram + tc_gram_at(npu, inrange ? p : 0, 0);
 
-    f.d0 = (inrange && i0 < n) ? gram[tc_gram_at(npu, p, tc_pidx(n, i0, i0))].x : 1.f;
-    f.d1 = (inrange && i1 < n) ? gram[tc_gram_at(npu, p, tc_pidx(n, i1, i1))].x : 1.f;
-#pragma unroll
-    for (int t = 0; t < 17; t++) {
-        const int q = g.gl + 16 * t;
-
-        f.ga[t] = (inrange && q < npu) ? gram[tc_gram_at(npu, p, q)] : make_float2(0.f, 0.f);
-    }
+    f.d0 = (inrange && i0 < n) ? sums[tc_pidx(n, i0, i0)].x : 1.f;
+    f.d1 = (inrange && i1 < n) ? sums[tc_pidx(n, i1, i1)].x : 1.f;
+    gram_batch(f.a, 0, npu, inrange, sums, g);
+    gram_batch(f.b, LT_BATCH, npu, inrange, sums, g);
 }
 
 /* T of the group's pixel from its packed Gram sums (tcoh.cl:611-636);
-   identity for an inactive group. The entries come in two batches of 17
-   (f, loaded ahead) and 16 per lane, each batch's loads issued before any
-   use (one batch of 33 held 66 registers through the processing and
-   spilled); upper_tab is the CTA's shared-memory copy of the packed-entry
-   table. */
+   identity for an inactive group. A loop over batches of LT_BATCH entries per
+   lane, the sums two batches ahead in flight: unrolled over all 33 entries the
+   code took 43 KB of the kernel's 200 KB of instructions that every pixel
+   goes through, more than the instruction caches hold (16 pixels at 30 dates:
+   18.2k -> 10.2k cycles of this stage). upper_tab is the CTA's shared-memory
+   copy of the packed-entry table. */
+template <bool EMI, bool ADJ>
 __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k, int p, bool active,
                        int looks, const float2 *__restrict__ gram, const TFirst &f,
                        const unsigned short *upper_tab, const HWs &w, int ld, const Pair &g,
@@ -1320,7 +1488,6 @@ __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
 {
     const int n = s.n, npu = tc_npu(n);
     const int i0 = g.gl, i1 = g.gl + 16;
-    float2 gb[16];
     const float d0 = active ? f.d0 : 1.f, d1 = active ? f.d1 : 1.f;
 
     if (i0 < n)
@@ -1328,14 +1495,30 @@ __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
     if (i1 < n)
         w.nrm[i1] = d1 > 0.f ? __frcp_rn(__fsqrt_rn(d1)) : 0.f;
     gsync(g);
-    load_T_batch<17>(f.ga, 0, n, npu, active, looks, k, upper_tab, w, ld, g, boundary);
-#pragma unroll
-    for (int t = 0; t < 16; t++) {
-        const int q = g.gl + 16 * (17 + t);
+    const float fl = (float)looks;
+    const bool debias = k.bias && looks > 1;
+    const float ilm1 = debias ? __frcp_rn(fl - 1.0f) : 0.f;
 
-        gb[t] = (active && q < npu) ? gram[tc_gram_at(npu, p, q)] : make_float2(0.f, 0.f);
+    const float2 *sums = gram + tc_gram_at(npu, p, 0);
+    float2 v[LT_BATCH], next[LT_BATCH];
+
+#pragma unroll
+    for (int u = 0; u < LT_BATCH; u++) {
+        v[u] = f.a[u];
+        next[u] = f.b[u];
     }
-    load_T_batch<16>(gb, 17, n, npu, active, looks, k, upper_tab, w, ld, g, boundary);
+#pragma unroll 1
+    for (int t0 = 0; 16 * t0 < npu; t0 += LT_BATCH) {
+        float2 after[LT_BATCH];
+
+        gram_batch(after, t0 + 2 * LT_BATCH, npu, active, sums, g);
+        load_T_batch<EMI, ADJ>(v, t0, npu, active, fl, ilm1, debias, upper_tab, w, ld, g, boundary);
+#pragma unroll
+        for (int u = 0; u < LT_BATCH; u++) {
+            v[u] = next[u];
+            next[u] = after[u];
+        }
+    }
     gsync(g);
     boundary = ((__ballot_sync(FULL, boundary) >> g.base) & 0xFFFFu) != 0u;
 }
@@ -1351,8 +1534,8 @@ __device__ bool linked16(int n, int ld, const float2 *T, const Pair &g)
 
     while (__any_sync(FULL, todo != 0u && reached != all)) {
         const int f = todo ? __ffs(todo) - 1 : 0;
-        const float2 a = i0 < n ? T[f * ld + i0] : make_float2(0.f, 0.f);
-        const float2 b = i1 < n ? T[f * ld + i1] : make_float2(0.f, 0.f);
+        const float2 a = i0 < n ? T[min(i0, f) * ld + max(i0, f)] : make_float2(0.f, 0.f);
+        const float2 b = i1 < n ? T[min(i1, f) * ld + max(i1, f)] : make_float2(0.f, 0.f);
         const unsigned lo = __ballot_sync(FULL, a.x != 0.f || a.y != 0.f) >> g.base;
         const unsigned hi = __ballot_sync(FULL, b.x != 0.f || b.y != 0.f) >> g.base;
         const unsigned nw = ((lo & 0xFFFFu) | (hi << 16)) & ~reached;
@@ -1414,6 +1597,7 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Pair &g, double2 z0d
     float sr = 0.f, si = 0.f;
     const int npu = tc_npu(n);
 
+#pragma unroll 4
     for (int q = g.gl; q < npu; q += 16) {
         const int i = upper_tab[q] >> 8, j = upper_tab[q] & 255;
 
@@ -1424,7 +1608,7 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Pair &g, double2 z0d
         float ur = 1.f, ui = 0.f;
 
         if (m2 > 0.f) {
-            const float r = rsqrtf(m2);
+            const float r = rsqrt_approx(m2);
 
             ur = tv.x * r;
             ui = tv.y * r;
@@ -1817,6 +2001,12 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
         s_upper[e] = upper_tab[e];
     __syncthreads();
 
+    if (EMI) {
+        for (int e = n * ld + g.gl; e < 32 * ld + 32; e += 16)
+            w.T[e] = make_float2(0.f, 0.f);
+        __syncthreads();
+    }
+
     /* The warps of a CTA take pixel pairs qb + warp and run each stage
        together, separated by CTA barriers: the stages' code is far larger
        than the instruction cache, and warps in different stages would keep
@@ -1870,7 +2060,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
         if (run) {
             bool boundary = false;
 
-            load_T(s, c, k, p, active, looks, gram, tf, s_upper, w, ld, g, boundary);
+            load_T<EMI, ADJ>(s, c, k, p, active, looks, gram, tf, s_upper, w, ld, g, boundary);
             if (queue && active && boundary) {
                 sent = true;
                 if (g.gl == 0)
@@ -1898,9 +2088,12 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
             gsync(g);
             if (!active) {
                 /* a well-conditioned stand-in keeps the group in step */
-                for (int r = g.gl; r < n; r += 16)
+                for (int r = g.gl; r < n; r += 16) {
                     for (int j = 0; j < n; j++)
                         w.T[r * ld + j] = make_float2(r == j ? 1.f : 0.f, 0.f);
+                    if (EMI)
+                        abs_slot(w, ld, r, r) = 1.0;
+                }
             }
             gsync(g);
             run = __any_sync(FULL, active);
@@ -1935,32 +2128,25 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
             __syncthreads();
         }
         else {
-            /* stage 2: |T|^-1 in double */
+            /* stage 2: |T|^-1 in double, M = |T|^-1 o T rounded to float */
             if (run)
-                st |= emi_inverse(n, ld, w, V, V + n * ld, V + 2 * n * ld, g, inv_max);
+                st |= emi_matrix<ADJ>(n, ld, w, V, V + n * ld, V + 2 * n * ld, g, inv_max);
             __syncthreads();
-            /* stage 3: M = |T|^-1 o T in float rows, Householder reduction */
+            /* stage 3: M's rows and their Householder reduction */
             if (run) {
+                const int ld = opaque(L.ld);
+
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
-                    r0[j] = make_float2(0.f, 0.f);
-                    r1[j] = make_float2(0.f, 0.f);
-                    if (j < n) {
-                        if (i0 < n) {
-                            const double2 m = mval(w, ld, i0, j);
+                    /* M_ij left of the diagonal, conj(M_ji) right of it */
+                    const float2 a = w.T[j >= 16 ? j * ld + i0 : TC_LOWER(i0, j)];
+                    const float2 b = w.T[j < 16 ? i1 * ld + j : TC_LOWER(i1, j)];
 
-                            r0[j] = make_float2((float)m.x, (float)m.y);
-                        }
-                        if (i1 < n) {
-                            const double2 m = mval(w, ld, i1, j);
-
-                            r1[j] = make_float2((float)m.x, (float)m.y);
-                        }
-                    }
+                    r0[j] = make_float2(a.x, j < 16 && i0 >= j ? a.y : -a.y);
+                    r1[j] = make_float2(b.x, j < 16 || i1 >= j ? b.y : -b.y);
                 }
                 gsync(g);
-                /* The reduction parks its vectors in T's lower triangle,
-                   which mval no longer reads (it takes T_ij from i < j). */
+                /* The reduction parks its vectors in T's lower triangle. */
                 householder(r0, r1, n, w, ld, g);
             }
             __syncthreads();
@@ -1981,8 +2167,16 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                    largest error over 896k pixels of the 30-date AD/EMI/-b
                    workload unchanged (3.4e-5) at 6 % less link time. */
                 if (active && sturm16(w.d, w.e2f, n, lambda + TC_REFINE_GAP * norm,
-                                      1.0e-30f + 1.0e-14f * norm) >= 2)
-                    refine(n, ld, w, alone(g), z0, z1, yr, piv);
+                                      1.0e-30f + 1.0e-14f * norm) >= 2) {
+#pragma unroll
+                    for (int k = 0; k < 32; k += 4)
+                        *(float4 *)(w.y + k) =
+                            make_float4(yr[k], yr[k + 1], yr[k + 2], yr[k + 3]);
+                    const double4 z = refine(n, ld, w, alone(g), z0, z1, piv);
+
+                    z0 = make_double2(z.x, z.y);
+                    z1 = make_double2(z.z, z.w);
+                }
                 /* Pixels whose gamma the float rounding of T may move by
                    more than ~1e-5 go to the exact tier: the first-order
                    sensitivity of M's eigenvector to T grows with
@@ -2067,10 +2261,13 @@ HalfLayout half_layout(int n, int emi, int adj = 0)
 
     L.n = n;
     L.ld = n | 1;
-    L.off_T = take(8 * n * L.ld);
+    /* EMI: rows from n to 31 stay zero; column indices up to 31 */
+    L.off_T = take(8 * (emi ? 32 * L.ld + 32 : n * L.ld));
     L.off_G = take(emi ? 8 * tc_npu(n) : 0);
-    /* stage-local: the sweep's pivot rows (inverse), the Householder
-       vectors (reduction) and the adjoint's vectors share one region */
+    /* stage-local: the reciprocal date norms (T), the sweep's pivot rows
+       (inverse), the Householder vectors (reduction), the solves' and the
+       refinement's vectors, and the phasors (gamma) share one region; the
+       adjoint keeps the norms and the phasors for its backward stage */
     L.off_vw = take(16 * 64);
     L.off_rs = L.off_vw;
     L.off_x = L.off_vw;
@@ -2078,14 +2275,16 @@ HalfLayout half_layout(int n, int emi, int adj = 0)
     L.off_tau = take(8 * 32);
     L.off_d = take(4 * 32);
     L.off_e = take(4 * 32);
-    L.off_df = take(4 * 32);
     L.off_e2f = take(4 * 32);
-    L.off_y = take(4 * 32);
-    L.off_nrm = take(4 * 32);
-    L.off_zs = take(8 * 32);
-    L.off_lam = 0;
+    L.off_nrm = adj ? take(4 * 32) : L.off_vw;
+    L.off_zs = adj ? take(8 * 32) : L.off_vw;
     L.off_Db = take(adj && emi ? 8 * n * L.ld : 0);
-    L.per_group = off;
+    /* the two halves of a warp read the same offsets of neighbouring
+       workspaces: 64 bytes apart modulo the banks, so that their broadcasts
+       and their rows of 16 floats fall into different ones (a broadcast of 8
+       bytes takes 1.06 cycles of the SM's shared memory then, and 2.0 with
+       both halves in the same banks) */
+    L.per_group = (off + 63) / 128 * 128 + 64;
     return L;
 }
 
