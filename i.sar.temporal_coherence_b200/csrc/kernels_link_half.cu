@@ -240,6 +240,7 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
     w.vw[48 + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
     StepHead hd = step_head(r0[0], r1[0], 0, n, g);
 
+#pragma unroll 1
     for (int k = 0; k < n - 1; k++) {
         const int len = n - 1 - k;
         const float2 c0 = r0[0], c1 = r1[0];
@@ -389,6 +390,7 @@ __device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, f
 {
     const int i0 = g.gl, i1 = g.gl + 16, nk = n - 1;
 
+#pragma unroll 1
     for (int b = 0; b < nk; b += 4) {
         float2 v0[4], v1[4], ta[4];
 
@@ -729,6 +731,7 @@ __device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g
 #pragma unroll
     for (int k = 0; k < 32; k++)
         yr[k] = 1.f;
+#pragma unroll 1
     for (int it = 0; it < 3; it++) {
         tri_solve(yr, f);
         float nrm = 0.f, odd = 0.f;
@@ -812,6 +815,7 @@ __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor,
     bool ok = fabs(r[0]) > floor;
     double id = rcp_newton(r[0]);
 
+#pragma unroll 1
     for (int k = 0; k < n; k++) {
         const bool piv0 = i0 == k, piv1 = i1 == k;
         /* the pivot row scales by 1 / a_kk: a_kj - (1 - 1 / a_kk) a_kj, with
@@ -1107,6 +1111,7 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
     load_abs(g0, g1, ld, w, pg);
     const bool swept = sweep16(g0, g1, n, 1.0e-5, w.rs, pg);
 
+#pragma unroll 1
     for (int k = n; k < 32; k++) {
         const double t0 = g0[0], t1 = g1[0];
 
