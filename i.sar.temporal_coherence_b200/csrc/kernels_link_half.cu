@@ -99,6 +99,22 @@ __device__ __forceinline__ T gsum(T v, const G &g)
 }
 
 template <class G>
+__device__ __forceinline__ float2 gsum2(float2 v, const G &g)
+{
+    /* the two sums level by level: shuffles keep their order, and one sum
+       after the other would wait twice as often */
+#pragma unroll
+    for (int o = 8; o; o >>= 1) {
+        const float x = __shfl_xor_sync(g.members(), v.x, o);
+        const float y = __shfl_xor_sync(g.members(), v.y, o);
+
+        v.x += x;
+        v.y += y;
+    }
+    return v;
+}
+
+template <class G>
 __device__ __forceinline__ float gmaxf(float v, const G &g)
 {
 #pragma unroll
@@ -193,26 +209,98 @@ __device__ __forceinline__ HWs hws(unsigned char *base, const HalfLayout &L)
 /* Householder reduction of the group's matrix (rows in r0, r1).       */
 /* ------------------------------------------------------------------ */
 
-/* Norm of the sub-pivot part of the pivot column, the sub-diagonal and the
-   diagonal of step k, from the pivot column values c0, c1 of rows i0, i1. */
+/* The hardware's approximate reciprocal, within two ulps; operands and results
+   are never denormal where it is used. */
+__device__ __forceinline__ float rcp_approx(float x)
+{
+    float y;
+
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+/* The approximate reciprocal square root, likewise. */
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float y;
+
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+/* 1 / x correctly rounded, by one Newton step with fused multiply-adds from the
+   approximate reciprocal (Markstein, IBM Journal of Research and Development
+   34, 1990), and the square root by his iteration from the approximate
+   reciprocal root. Equal to __frcp_rn and sqrtf for every significand and
+   every exponent from -90 to 90 (all of them compared); the caller keeps to
+   exponents within 80. They have no branches: with the intrinsics a
+   Householder step took 17 % longer (2.48k against 2.14k cycles, eight warps,
+   30 dates). */
+__device__ __forceinline__ float rcp_rn(float x)
+{
+    const float y = rcp_approx(x);
+
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+
+__device__ __forceinline__ float sqrt_rn(float a)
+{
+    const float y = rsqrt_approx(a);
+    float s = __fmul_rn(a, y), h = 0.5f * y;
+    const float e = fmaf(-s, h, 0.5f);
+
+    h = fmaf(h, e, h);
+    s = fmaf(s, e, s);
+    return fmaf(fmaf(-s, s, a), h, s);
+}
+
+/* Fused products with the roundings written out, so that what a pixel gets does
+   not depend on how the compiler contracts the expressions around them. */
+__device__ __forceinline__ float2 cscale(float2 a, float2 b) /* a b */
+{
+    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y)));
+}
+
+/* What step k needs of its pivot column: the sub-diagonal beta that it leaves,
+   the diagonal, tau, and the scale that makes the column v (v = column * scale
+   below row k + 1, 1 in row k + 1; the column itself where tau = 0). */
 struct StepHead {
-    float xn2;
-    float2 alpha;
-    float dk;
+    float beta, dk;
+    float2 tau, scale;
 };
 
-__device__ __forceinline__ StepHead step_head(float2 c0, float2 c1, int k, int n, const Pair &g)
+/* From the sub-diagonal element alpha and the squared norm xn2 below it. */
+__device__ __forceinline__ void reflector(StepHead &h, float2 alpha, float xn2)
+{
+    const bool zero = xn2 == 0.f && alpha.y == 0.f;
+    const float s2 = __fadd_rn(fmaf(alpha.x, alpha.x, __fmul_rn(alpha.y, alpha.y)), xn2);
+    float beta = -copysignf(sqrt_rn(s2), alpha.x), ib = rcp_rn(beta);
+    float dr = alpha.x - beta, di = alpha.y;
+    float iden = rcp_rn(fmaf(di, di, __fmul_rn(dr, dr)));
+
+    if (__any_sync(FULL, !zero && !(s2 > 1.0e-24f && s2 < 1.0e24f))) {
+        /* columns near the ends of the float range: rarely, if ever */
+        beta = -copysignf(sqrtf(s2), alpha.x);
+        ib = __frcp_rn(beta);
+        dr = alpha.x - beta;
+        iden = __frcp_rn(fmaf(di, di, __fmul_rn(dr, dr)));
+    }
+    h.beta = zero ? alpha.x : beta;
+    h.tau = zero ? make_float2(0.f, 0.f)
+                 : make_float2(__fmul_rn(beta - alpha.x, ib), __fmul_rn(-alpha.y, ib));
+    h.scale = make_float2(__fmul_rn(dr, iden), __fmul_rn(-di, iden));
+    if (h.tau.x == 0.f && h.tau.y == 0.f)
+        h.scale = make_float2(1.f, 0.f);
+}
+
+/* The lane's part of that norm for step k, of rows i0, i1. */
+__device__ __forceinline__ float below(float2 c0, float2 c1, int k, int n, const Pair &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
-    StepHead h;
-    float x = (i0 >= k + 2 && i0 < n ? c0.x * c0.x + c0.y * c0.y : 0.f) +
-              (i1 >= k + 2 && i1 < n ? c1.x * c1.x + c1.y * c1.y : 0.f);
-    const float2 sa = k + 1 < 16 ? c0 : c1;
+    const float a = fmaf(c0.x, c0.x, __fmul_rn(c0.y, c0.y));
+    const float b = fmaf(c1.x, c1.x, __fmul_rn(c1.y, c1.y));
 
-    h.alpha = make_float2(gbcast(sa.x, k + 1, g), gbcast(sa.y, k + 1, g));
-    h.dk = gbcast(k < 16 ? c0.x : c1.x, k, g);
-    h.xn2 = gsum(x, g);
-    return h;
+    return __fadd_rn(i0 >= k + 2 && i0 < n ? a : 0.f, i1 >= k + 2 && i1 < n ? b : 0.f);
 }
 
 /* One element of the rank-2 update: t - (v conj(wj) + w conj(vj)), with
@@ -230,6 +318,15 @@ __device__ __forceinline__ float2 r2(float2 t, float2 nv, float2 nw, float4 q)
     return t;
 }
 
+/* Householder reduction of the group's matrix to real tridiagonal form, its
+   columns 0 .. n - 1 in r0, r1; at step k the pivot column is r[0]. A step is
+   one chain: v to memory and back, A v, two sums over the group, w to memory
+   and back, the next pivot column, the sum of its squares, a square root and
+   two reciprocals. The latter run between the blocks of the rank-2 update of
+   the other columns, which does not need them. Two warps per scheduler do not
+   hide the chain: 2.14k cycles a step at 30 dates for 1.1k of instructions
+   issued (2.82k with the square root ahead of the step, branches for v, the
+   intrinsics' divisions and one sum after the other). */
 __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs &w, int ld,
                             const Pair &g)
 {
@@ -238,136 +335,131 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
     /* Entries 32..63 stay zero: whole blocks of 4 columns may run past n. */
     w.vw[32 + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
     w.vw[48 + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
-    StepHead hd = step_head(r0[0], r1[0], 0, n, g);
+    StepHead h;
+    {
+        const float2 a = make_float2(gbcast(r0[0].x, 1, g), gbcast(r0[0].y, 1, g));
+
+        h.dk = gbcast(r0[0].x, 0, g);
+        reflector(h, a, gsum(below(r0[0], r1[0], 0, n, g), g));
+    }
+    /* diagonal, sub-diagonal and tau of steps gl and gl + 16 */
+    float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
 
 #pragma unroll 1
     for (int k = 0; k < n - 1; k++) {
         const int len = n - 1 - k;
-        const float2 c0 = r0[0], c1 = r1[0];
-        const float2 alpha = hd.alpha;
-        const float xn2 = hd.xn2;
-        float beta, tr = 0.f, ti = 0.f, sr = 0.f, si = 0.f;
+        const float2 tau = h.tau;
+        float2 v0 = cscale(r0[0], h.scale), v1 = cscale(r1[0], h.scale);
 
-        if (xn2 == 0.f && alpha.y == 0.f)
-            beta = alpha.x;
-        else {
-            beta = -copysignf(sqrtf(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
-            const float ib = __frcp_rn(beta);
-
-            tr = (beta - alpha.x) * ib;
-            ti = -alpha.y * ib;
-            const float dr = alpha.x - beta, di = alpha.y;
-            const float iden = __frcp_rn(dr * dr + di * di);
-
-            sr = dr * iden;
-            si = -di * iden;
-        }
-        const bool refl = !(tr == 0.f && ti == 0.f);
-        float2 v0 = make_float2(0.f, 0.f), v1 = make_float2(0.f, 0.f);
-
-        if (i0 == k + 1)
-            v0 = make_float2(1.f, 0.f);
-        else if (i0 > k + 1 && i0 < n)
-            v0 = refl ? make_float2(c0.x * sr - c0.y * si, c0.x * si + c0.y * sr) : c0;
-        if (i1 == k + 1)
-            v1 = make_float2(1.f, 0.f);
-        else if (i1 > k + 1 && i1 < n)
-            v1 = refl ? make_float2(c1.x * sr - c1.y * si, c1.x * si + c1.y * sr) : c1;
-        if (i0 > k && i0 < n)
-            w.T[i0 * ld + k] = v0;
-        if (i1 > k && i1 < n)
-            w.T[i1 * ld + k] = v1;
-        if (g.gl == 0) {
-            w.d[k] = hd.dk;
-            w.e[k] = beta;
-            w.tau[k] = make_float2(tr, ti);
-        }
+        v0.x = i0 > k + 1 && i0 < n ? v0.x : i0 == k + 1 ? 1.f : 0.f;
+        v0.y = i0 > k + 1 && i0 < n ? v0.y : 0.f;
+        v1.x = i1 > k + 1 && i1 < n ? v1.x : i1 == k + 1 ? 1.f : 0.f;
+        v1.y = i1 > k + 1 && i1 < n ? v1.y : 0.f;
         /* With tau = 0 the update below is an exact zero: only the shift. */
         ((float2 *)w.vw)[2 * i0] = v0;
         ((float2 *)w.vw)[2 * i1] = v1;
         gsync(g);
         const float4 *vwk = w.vw + k;
         float2 p0a = make_float2(0.f, 0.f), p0b = p0a, p1a = p0a, p1b = p0a;
-
+        if (g.gl == (k & 15)) {
+            if (k < 16)
+                s0 = make_float4(h.dk, h.beta, tau.x, tau.y);
+            else
+                s1 = make_float4(h.dk, h.beta, tau.x, tau.y);
+        }
 #pragma unroll
         for (int jb = 1; jb < 32; jb += 4) {
             if (jb > len)
                 break;
 #pragma unroll
             for (int jj = jb; jj < jb + 4 && jj < 32; jj++) {
-                const float2 vj = *(const float2 *)&vwk[jj];
+                const float2 v = *(const float2 *)&vwk[jj];
                 float2 &q0 = (jj & 1) ? p0b : p0a;
                 float2 &q1 = (jj & 1) ? p1b : p1a;
 
-                q0.x = fmaf(r0[jj].x, vj.x, fmaf(-r0[jj].y, vj.y, q0.x));
-                q0.y = fmaf(r0[jj].x, vj.y, fmaf(r0[jj].y, vj.x, q0.y));
-                q1.x = fmaf(r1[jj].x, vj.x, fmaf(-r1[jj].y, vj.y, q1.x));
-                q1.y = fmaf(r1[jj].x, vj.y, fmaf(r1[jj].y, vj.x, q1.y));
+                q0.x = fmaf(r0[jj].x, v.x, fmaf(-r0[jj].y, v.y, q0.x));
+                q0.y = fmaf(r0[jj].x, v.y, fmaf(r0[jj].y, v.x, q0.y));
+                q1.x = fmaf(r1[jj].x, v.x, fmaf(-r1[jj].y, v.y, q1.x));
+                q1.y = fmaf(r1[jj].x, v.y, fmaf(r1[jj].y, v.x, q1.y));
             }
         }
         const float2 p0 = make_float2(p0a.x + p0b.x, p0a.y + p0b.y);
         const float2 p1 = make_float2(p1a.x + p1b.x, p1a.y + p1b.y);
-        float2 w0 = make_float2(tr * p0.x - ti * p0.y, tr * p0.y + ti * p0.x);
-        float2 w1 = make_float2(tr * p1.x - ti * p1.y, tr * p1.y + ti * p1.x);
-        float pr = (i0 > k ? w0.x * v0.x + w0.y * v0.y : 0.f) +
-                   (i1 > k ? w1.x * v1.x + w1.y * v1.y : 0.f);
-        float pi = (i0 > k ? w0.x * v0.y - w0.y * v0.x : 0.f) +
-                   (i1 > k ? w1.x * v1.y - w1.y * v1.x : 0.f);
+        float2 w0 = make_float2(fmaf(tau.x, p0.x, -__fmul_rn(tau.y, p0.y)),
+                                fmaf(tau.y, p0.x, __fmul_rn(tau.x, p0.y)));
+        float2 w1 = make_float2(fmaf(tau.x, p1.x, -__fmul_rn(tau.y, p1.y)),
+                                fmaf(tau.y, p1.x, __fmul_rn(tau.x, p1.y)));
+        /* (w^H v) */
+        float2 pp;
+        {
+            const float ax = fmaf(w0.x, v0.x, __fmul_rn(w0.y, v0.y));
+            const float ay = fmaf(w0.x, v0.y, -__fmul_rn(w0.y, v0.x));
+            const float bx = fmaf(w1.x, v1.x, __fmul_rn(w1.y, v1.y));
+            const float by = fmaf(w1.x, v1.y, -__fmul_rn(w1.y, v1.x));
 
-        pr = gsum(pr, g);
-        pi = gsum(pi, g);
-        const float hr = -0.5f * (tr * pr - ti * pi), hi = -0.5f * (tr * pi + ti * pr);
+            pp.x = __fadd_rn(i0 > k ? ax : 0.f, i1 > k ? bx : 0.f);
+            pp.y = __fadd_rn(i0 > k ? ay : 0.f, i1 > k ? by : 0.f);
+        }
+        pp = gsum2(pp, g);
+        const float hr = -0.5f * fmaf(tau.x, pp.x, -__fmul_rn(tau.y, pp.y));
+        const float hi = -0.5f * fmaf(tau.y, pp.x, __fmul_rn(tau.x, pp.y));
 
-        w0.x += hr * v0.x - hi * v0.y;
-        w0.y += hr * v0.y + hi * v0.x;
-        w1.x += hr * v1.x - hi * v1.y;
-        w1.y += hr * v1.y + hi * v1.x;
-        if (i0 <= k)
-            w0 = make_float2(0.f, 0.f);
-        if (i1 <= k)
-            w1 = make_float2(0.f, 0.f);
+        w0.x = i0 > k ? __fadd_rn(w0.x, fmaf(hr, v0.x, -__fmul_rn(hi, v0.y))) : 0.f;
+        w0.y = i0 > k ? __fadd_rn(w0.y, fmaf(hr, v0.y, __fmul_rn(hi, v0.x))) : 0.f;
+        w1.x = i1 > k ? __fadd_rn(w1.x, fmaf(hr, v1.x, -__fmul_rn(hi, v1.y))) : 0.f;
+        w1.y = i1 > k ? __fadd_rn(w1.y, fmaf(hr, v1.y, __fmul_rn(hi, v1.x))) : 0.f;
         ((float2 *)w.vw)[2 * i0 + 1] = w0;
         ((float2 *)w.vw)[2 * i1 + 1] = w1;
         gsync(g);
+        if (i0 > k && i0 < n)
+            w.T[i0 * ld + k] = v0;
+        if (i1 > k && i1 < n)
+            w.T[i1 * ld + k] = v1;
         const float2 nv0 = make_float2(-v0.x, -v0.y), nv1 = make_float2(-v1.x, -v1.y);
         const float2 nw0 = make_float2(-w0.x, -w0.y), nw1 = make_float2(-w1.x, -w1.y);
 
-        /* Column k + 1 first: it is the next pivot column, so the next
-           step's reductions overlap the rest of this update. */
+        /* Column k + 1 first, the next pivot column. */
         {
-            const float4 q = vwk[1];
+            const float4 q1 = vwk[1];
 
-            r0[0] = r2(r0[1], nv0, nw0, q);
-            r1[0] = r2(r1[1], nv1, nw1, q);
+            r0[0] = r2(r0[1], nv0, nw0, q1);
+            r1[0] = r2(r1[1], nv1, nw1, q1);
         }
-        hd = step_head(r0[0], r1[0], k + 1, n, g); /* unused after the last step */
-#pragma unroll
-        for (int jj = 2; jj < 6; jj++) {
-            const float4 q = vwk[jj];
+        const float2 na = k + 2 < 16 ? r0[0] : r1[0];
+        const float2 alpha = make_float2(gbcast(na.x, k + 2, g), gbcast(na.y, k + 2, g));
+        float x = below(r0[0], r1[0], k + 1, n, g); /* unused after the last step */
 
-            r0[jj - 1] = r2(r0[jj], nv0, nw0, q);
-            r1[jj - 1] = r2(r1[jj], nv1, nw1, q);
-        }
+        h.dk = gbcast(k + 1 < 16 ? r0[0].x : r1[0].x, k + 1, g);
 #pragma unroll
-        for (int jb = 6; jb < 32; jb += 4) {
-            if (jb > len)
-                break;
+        for (int jb = 2; jb < 32; jb += 4) {
+            if (jb == 2 || jb <= len) {
 #pragma unroll
-            for (int jj = jb; jj < jb + 4 && jj < 32; jj++) {
-                const float4 q = vwk[jj];
+                for (int jj = jb; jj < jb + 4 && jj < 32; jj++) {
+                    const float4 q = vwk[jj];
 
-                r0[jj - 1] = r2(r0[jj], nv0, nw0, q);
-                r1[jj - 1] = r2(r1[jj], nv1, nw1, q);
+                    r0[jj - 1] = r2(r0[jj], nv0, nw0, q);
+                    r1[jj - 1] = r2(r1[jj], nv1, nw1, q);
+                }
             }
+            if (jb <= 14)
+                x += __shfl_xor_sync(FULL, x, 16 >> ((jb + 2) / 4));
+            else if (jb == 18)
+                reflector(h, alpha, x);
         }
         gsync(g);
     }
-    {
-        const float dl = gbcast(n - 1 < 16 ? r0[0].x : r1[0].x, n - 1, g);
-
-        if (g.gl == 0)
-            w.d[n - 1] = dl;
+    if (g.gl < n - 1) {
+        w.d[g.gl] = s0.x;
+        w.e[g.gl] = s0.y;
+        w.tau[g.gl] = make_float2(s0.z, s0.w);
     }
+    if (g.gl + 16 < n - 1) {
+        w.d[g.gl + 16] = s1.x;
+        w.e[g.gl + 16] = s1.y;
+        w.tau[g.gl + 16] = make_float2(s1.z, s1.w);
+    }
+    if (g.gl == 0)
+        w.d[n - 1] = h.dk;
     gsync(g);
 }
 
@@ -495,25 +587,6 @@ __device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, f
     }
 }
 
-
-/* The hardware's approximate reciprocal, within two ulps; operands and results
-   are never denormal where it is used. */
-__device__ __forceinline__ float rcp_approx(float x)
-{
-    float y;
-
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-/* The approximate reciprocal square root, likewise. */
-__device__ __forceinline__ float rsqrt_approx(float x)
-{
-    float y;
-
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 /* Eigenvalues of the group's tridiagonal below x. The chain from one pivot to
    the next is a reciprocal, a select and a fused multiply-add: the test for a
