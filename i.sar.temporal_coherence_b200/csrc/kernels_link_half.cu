@@ -29,7 +29,7 @@
  * Elsewhere the float eigen-solve adds less to gamma's error than the float
  * coherence sums do.
  */
-#include "tcoh_internal.h"
+#include "link_float.cuh"
 
 #include <math.h>
 
@@ -209,58 +209,6 @@ __device__ __forceinline__ HWs hws(unsigned char *base, const HalfLayout &L)
 /* Householder reduction of the group's matrix (rows in r0, r1).       */
 /* ------------------------------------------------------------------ */
 
-/* The hardware's approximate reciprocal, within two ulps; operands and results
-   are never denormal where it is used. */
-__device__ __forceinline__ float rcp_approx(float x)
-{
-    float y;
-
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-/* The approximate reciprocal square root, likewise. */
-__device__ __forceinline__ float rsqrt_approx(float x)
-{
-    float y;
-
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-/* 1 / x correctly rounded, by one Newton step with fused multiply-adds from the
-   approximate reciprocal (Markstein, IBM Journal of Research and Development
-   34, 1990), and the square root by his iteration from the approximate
-   reciprocal root. Equal to __frcp_rn and sqrtf for every significand and
-   every exponent from -90 to 90 (all of them compared); the caller keeps to
-   exponents within 80. They have no branches: with the intrinsics a
-   Householder step took 17 % longer (2.48k against 2.14k cycles, eight warps,
-   30 dates). */
-__device__ __forceinline__ float rcp_rn(float x)
-{
-    const float y = rcp_approx(x);
-
-    return fmaf(y, fmaf(-x, y, 1.0f), y);
-}
-
-__device__ __forceinline__ float sqrt_rn(float a)
-{
-    const float y = rsqrt_approx(a);
-    float s = __fmul_rn(a, y), h = 0.5f * y;
-    const float e = fmaf(-s, h, 0.5f);
-
-    h = fmaf(h, e, h);
-    s = fmaf(s, e, s);
-    return fmaf(fmaf(-s, s, a), h, s);
-}
-
-/* Fused products with the roundings written out, so that what a pixel gets does
-   not depend on how the compiler contracts the expressions around them. */
-__device__ __forceinline__ float2 cscale(float2 a, float2 b) /* a b */
-{
-    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y)));
-}
-
 /* What step k needs of its pivot column: the sub-diagonal beta that it leaves,
    the diagonal, tau, and the scale that makes the column v (v = column * scale
    below row k + 1, 1 in row k + 1; the column itself where tau = 0). */
@@ -301,21 +249,6 @@ __device__ __forceinline__ float below(float2 c0, float2 c1, int k, int n, const
     const float b = fmaf(c1.x, c1.x, __fmul_rn(c1.y, c1.y));
 
     return __fadd_rn(i0 >= k + 2 && i0 < n ? a : 0.f, i1 >= k + 2 && i1 < n ? b : 0.f);
-}
-
-/* One element of the rank-2 update: t - (v conj(wj) + w conj(vj)), with
-   nv = -v and nw = -w (four FMAs per component). */
-__device__ __forceinline__ float2 r2(float2 t, float2 nv, float2 nw, float4 q)
-{
-    t.x = fmaf(nv.x, q.z, t.x);
-    t.x = fmaf(nv.y, q.w, t.x);
-    t.x = fmaf(nw.x, q.x, t.x);
-    t.x = fmaf(nw.y, q.y, t.x);
-    t.y = fmaf(nv.y, q.z, t.y);
-    t.y = fmaf(-nv.x, q.w, t.y);
-    t.y = fmaf(nw.y, q.x, t.y);
-    t.y = fmaf(-nw.x, q.y, t.y);
-    return t;
 }
 
 /* Householder reduction of the group's matrix to real tridiagonal form, its
@@ -1136,15 +1069,6 @@ __device__ __noinline__ unsigned emi_fallback(int n, int ld, HWs w, double *A, d
    on and rows i1 >= 16 left of it up to column 15; only the diagonal blocks
    select. EMI's T has 32 rows, those from n on zero, so that entries beyond n
    need no test. */
-/* A value that the compiler cannot follow: the addresses formed from it are
-   not kept in registers from one pixel pair to the next (there are more of
-   them than registers; they would be spilled). */
-__device__ __forceinline__ int opaque(int v)
-{
-    asm volatile("" : "+r"(v));
-    return v;
-}
-
 #define TC_LOWER(i, j) ((i) > (j) ? (i) * ld + (j) : (j) * ld + (i))
 
 /* Rows i0, i1 of |T| from the slots that load_T filled. */

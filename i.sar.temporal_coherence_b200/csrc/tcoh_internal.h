@@ -294,6 +294,11 @@ cudaError_t tc_launch_link_half(const TcStrip &s, const TcChunk &c, const TcLink
                                 double *scratch, float *coh, float *pairs, float *phases,
                                 unsigned char *status, int *queue, int qstride, int sms,
                                 cudaStream_t st);
+cudaError_t tc_launch_link_wide(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
+                                const float2 *gram, const uint32_t *mask, const int *count,
+                                const unsigned short *upper_tab, const unsigned short *pair_tab,
+                                float *coh, float *pairs, float *phases, unsigned char *status,
+                                int *queue, int qstride, int sms, cudaStream_t st);
 size_t tc_link_half_scratch_bytes(int n, int sms);
 /* The link stage with the adjoint (n <= 32): gamma into coh, and into gbar
    (layout of gram) the gradient of gamma with respect to each pixel's
