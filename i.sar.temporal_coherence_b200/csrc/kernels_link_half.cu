@@ -31,6 +31,10 @@
  */
 #include "link_float.cuh"
 
+#ifndef TC_LINK_COLS
+#define TC_LINK_COLS 32
+#endif
+
 #include <math.h>
 
 #define FULL 0xffffffffu
@@ -48,6 +52,11 @@
 
 namespace {
 
+/* Columns (and rows) of the matrices in registers: 32, two rows per lane, or, in
+   kernels_link_half16.cu, 16, one row per lane (TWO false: the second row's
+   work is not compiled). */
+constexpr int NC = TC_LINK_COLS;
+constexpr bool TWO = NC == 32;
 constexpr int LT_BATCH = 6; /* entries of T per lane and turn of load_T */
 
 /* A half-warp. Collectives take their mask from members(): Pair, for code
@@ -248,7 +257,7 @@ __device__ __forceinline__ float below(float2 c0, float2 c1, int k, int n, const
     const float a = fmaf(c0.x, c0.x, __fmul_rn(c0.y, c0.y));
     const float b = fmaf(c1.x, c1.x, __fmul_rn(c1.y, c1.y));
 
-    return __fadd_rn(i0 >= k + 2 && i0 < n ? a : 0.f, i1 >= k + 2 && i1 < n ? b : 0.f);
+    return __fadd_rn(i0 >= k + 2 && i0 < n ? a : 0.f, TWO && i1 >= k + 2 && i1 < n ? b : 0.f);
 }
 
 /* Householder reduction of the group's matrix to real tridiagonal form, its
@@ -260,14 +269,15 @@ __device__ __forceinline__ float below(float2 c0, float2 c1, int k, int n, const
    hide the chain: 2.14k cycles a step at 30 dates for 1.1k of instructions
    issued (2.82k with the square root ahead of the step, branches for v, the
    intrinsics' divisions and one sum after the other). */
-__device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs &w, int ld,
+__device__ void householder(float2 (&r0)[NC], float2 (&r1)[NC], int n, const HWs &w, int ld,
                             const Pair &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
 
-    /* Entries 32..63 stay zero: whole blocks of 4 columns may run past n. */
-    w.vw[32 + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
-    w.vw[48 + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
+    /* Entries from NC on stay zero: whole blocks of 4 columns may run past n. */
+    w.vw[NC + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (TWO)
+        w.vw[NC + 16 + g.gl] = make_float4(0.f, 0.f, 0.f, 0.f);
     StepHead h;
     {
         const float2 a = make_float2(gbcast(r0[0].x, 1, g), gbcast(r0[0].y, 1, g));
@@ -282,38 +292,44 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
     for (int k = 0; k < n - 1; k++) {
         const int len = n - 1 - k;
         const float2 tau = h.tau;
-        float2 v0 = cscale(r0[0], h.scale), v1 = cscale(r1[0], h.scale);
+        float2 v0 = cscale(r0[0], h.scale), v1 = make_float2(0.f, 0.f);
+
+        if (TWO)
+            v1 = cscale(r1[0], h.scale);
 
         v0.x = i0 > k + 1 && i0 < n ? v0.x : i0 == k + 1 ? 1.f : 0.f;
         v0.y = i0 > k + 1 && i0 < n ? v0.y : 0.f;
-        v1.x = i1 > k + 1 && i1 < n ? v1.x : i1 == k + 1 ? 1.f : 0.f;
-        v1.y = i1 > k + 1 && i1 < n ? v1.y : 0.f;
+        v1.x = TWO && i1 > k + 1 && i1 < n ? v1.x : TWO && i1 == k + 1 ? 1.f : 0.f;
+        v1.y = TWO && i1 > k + 1 && i1 < n ? v1.y : 0.f;
         /* With tau = 0 the update below is an exact zero: only the shift. */
         ((float2 *)w.vw)[2 * i0] = v0;
-        ((float2 *)w.vw)[2 * i1] = v1;
+        if (TWO)
+            ((float2 *)w.vw)[2 * i1] = v1;
         gsync(g);
         const float4 *vwk = w.vw + k;
         float2 p0a = make_float2(0.f, 0.f), p0b = p0a, p1a = p0a, p1b = p0a;
         if (g.gl == (k & 15)) {
-            if (k < 16)
+            if (!TWO || k < 16)
                 s0 = make_float4(h.dk, h.beta, tau.x, tau.y);
             else
                 s1 = make_float4(h.dk, h.beta, tau.x, tau.y);
         }
 #pragma unroll
-        for (int jb = 1; jb < 32; jb += 4) {
+        for (int jb = 1; jb < NC; jb += 4) {
             if (jb > len)
                 break;
 #pragma unroll
-            for (int jj = jb; jj < jb + 4 && jj < 32; jj++) {
+            for (int jj = jb; jj < jb + 4 && jj < NC; jj++) {
                 const float2 v = *(const float2 *)&vwk[jj];
                 float2 &q0 = (jj & 1) ? p0b : p0a;
                 float2 &q1 = (jj & 1) ? p1b : p1a;
 
                 q0.x = fmaf(r0[jj].x, v.x, fmaf(-r0[jj].y, v.y, q0.x));
                 q0.y = fmaf(r0[jj].x, v.y, fmaf(r0[jj].y, v.x, q0.y));
-                q1.x = fmaf(r1[jj].x, v.x, fmaf(-r1[jj].y, v.y, q1.x));
-                q1.y = fmaf(r1[jj].x, v.y, fmaf(r1[jj].y, v.x, q1.y));
+                if (TWO) {
+                    q1.x = fmaf(r1[jj].x, v.x, fmaf(-r1[jj].y, v.y, q1.x));
+                    q1.y = fmaf(r1[jj].x, v.y, fmaf(r1[jj].y, v.x, q1.y));
+                }
             }
         }
         const float2 p0 = make_float2(p0a.x + p0b.x, p0a.y + p0b.y);
@@ -330,8 +346,8 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
             const float bx = fmaf(w1.x, v1.x, __fmul_rn(w1.y, v1.y));
             const float by = fmaf(w1.x, v1.y, -__fmul_rn(w1.y, v1.x));
 
-            pp.x = __fadd_rn(i0 > k ? ax : 0.f, i1 > k ? bx : 0.f);
-            pp.y = __fadd_rn(i0 > k ? ay : 0.f, i1 > k ? by : 0.f);
+            pp.x = __fadd_rn(i0 > k ? ax : 0.f, TWO && i1 > k ? bx : 0.f);
+            pp.y = __fadd_rn(i0 > k ? ay : 0.f, TWO && i1 > k ? by : 0.f);
         }
         pp = gsum2(pp, g);
         const float hr = -0.5f * fmaf(tau.x, pp.x, -__fmul_rn(tau.y, pp.y));
@@ -339,14 +355,15 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
 
         w0.x = i0 > k ? __fadd_rn(w0.x, fmaf(hr, v0.x, -__fmul_rn(hi, v0.y))) : 0.f;
         w0.y = i0 > k ? __fadd_rn(w0.y, fmaf(hr, v0.y, __fmul_rn(hi, v0.x))) : 0.f;
-        w1.x = i1 > k ? __fadd_rn(w1.x, fmaf(hr, v1.x, -__fmul_rn(hi, v1.y))) : 0.f;
-        w1.y = i1 > k ? __fadd_rn(w1.y, fmaf(hr, v1.y, __fmul_rn(hi, v1.x))) : 0.f;
+        w1.x = TWO && i1 > k ? __fadd_rn(w1.x, fmaf(hr, v1.x, -__fmul_rn(hi, v1.y))) : 0.f;
+        w1.y = TWO && i1 > k ? __fadd_rn(w1.y, fmaf(hr, v1.y, __fmul_rn(hi, v1.x))) : 0.f;
         ((float2 *)w.vw)[2 * i0 + 1] = w0;
-        ((float2 *)w.vw)[2 * i1 + 1] = w1;
+        if (TWO)
+            ((float2 *)w.vw)[2 * i1 + 1] = w1;
         gsync(g);
         if (i0 > k && i0 < n)
             w.T[i0 * ld + k] = v0;
-        if (i1 > k && i1 < n)
+        if (TWO && i1 > k && i1 < n)
             w.T[i1 * ld + k] = v1;
         const float2 nv0 = make_float2(-v0.x, -v0.y), nv1 = make_float2(-v1.x, -v1.y);
         const float2 nw0 = make_float2(-w0.x, -w0.y), nw1 = make_float2(-w1.x, -w1.y);
@@ -356,27 +373,29 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
             const float4 q1 = vwk[1];
 
             r0[0] = r2(r0[1], nv0, nw0, q1);
-            r1[0] = r2(r1[1], nv1, nw1, q1);
+            if (TWO)
+                r1[0] = r2(r1[1], nv1, nw1, q1);
         }
-        const float2 na = k + 2 < 16 ? r0[0] : r1[0];
+        const float2 na = !TWO || k + 2 < 16 ? r0[0] : r1[0];
         const float2 alpha = make_float2(gbcast(na.x, k + 2, g), gbcast(na.y, k + 2, g));
         float x = below(r0[0], r1[0], k + 1, n, g); /* unused after the last step */
 
-        h.dk = gbcast(k + 1 < 16 ? r0[0].x : r1[0].x, k + 1, g);
+        h.dk = gbcast(!TWO || k + 1 < 16 ? r0[0].x : r1[0].x, k + 1, g);
 #pragma unroll
-        for (int jb = 2; jb < 32; jb += 4) {
+        for (int jb = 2; jb < NC; jb += 4) {
             if (jb == 2 || jb <= len) {
 #pragma unroll
-                for (int jj = jb; jj < jb + 4 && jj < 32; jj++) {
+                for (int jj = jb; jj < jb + 4 && jj < NC; jj++) {
                     const float4 q = vwk[jj];
 
                     r0[jj - 1] = r2(r0[jj], nv0, nw0, q);
-                    r1[jj - 1] = r2(r1[jj], nv1, nw1, q);
+                    if (TWO)
+                        r1[jj - 1] = r2(r1[jj], nv1, nw1, q);
                 }
             }
             if (jb <= 14)
                 x += __shfl_xor_sync(FULL, x, 16 >> ((jb + 2) / 4));
-            else if (jb == 18)
+            if (jb == (TWO ? 18 : 14))
                 reflector(h, alpha, x);
         }
         gsync(g);
@@ -386,7 +405,7 @@ __device__ void householder(float2 (&r0)[32], float2 (&r1)[32], int n, const HWs
         w.e[g.gl] = s0.y;
         w.tau[g.gl] = make_float2(s0.z, s0.w);
     }
-    if (g.gl + 16 < n - 1) {
+    if (TWO && g.gl + 16 < n - 1) {
         w.d[g.gl + 16] = s1.x;
         w.e[g.gl + 16] = s1.y;
         w.tau[g.gl + 16] = make_float2(s1.z, s1.w);
@@ -427,7 +446,7 @@ __device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, f
 
             ta[m] = adjoint ? make_float2(t.x, -t.y) : t;
             v0[m] = ok && i0 > k && i0 < n ? w.T[i0 * ld + k] : make_float2(0.f, 0.f);
-            v1[m] = ok && i1 > k && i1 < n ? w.T[i1 * ld + k] : make_float2(0.f, 0.f);
+            v1[m] = TWO && ok && i1 > k && i1 < n ? w.T[i1 * ld + k] : make_float2(0.f, 0.f);
         }
         /* r[2m], r[2m+1]: v_m^H x; r[8 + 2p], r[9 + 2p]: v_m^H v_j, pairs
            p = (1,0), (2,0), (2,1), (3,0), (3,1), (3,2) */
@@ -514,8 +533,10 @@ __device__ void apply_q(int n, int ld, const HWs &w, const G &g, bool adjoint, f
         for (int m = 0; m < 4; m++) {
             x0.x -= v0[m].x * h[m].x - v0[m].y * h[m].y;
             x0.y -= v0[m].x * h[m].y + v0[m].y * h[m].x;
-            x1.x -= v1[m].x * h[m].x - v1[m].y * h[m].y;
-            x1.y -= v1[m].x * h[m].y + v1[m].y * h[m].x;
+            if (TWO) {
+                x1.x -= v1[m].x * h[m].x - v1[m].y * h[m].y;
+                x1.y -= v1[m].x * h[m].y + v1[m].y * h[m].x;
+            }
         }
     }
 }
@@ -615,17 +636,17 @@ __device__ float tri_eigenvalue(int n, int index, const HWs &w, const Pair &g, f
    and the shorter chain of sturm16: link stage 94.4 -> 85.7 ms per 512 x 4096
    AD / EMI / -b strip at 30 dates. */
 struct TriLU {
-    float rd[32], u1[32], u2[32], l[32]; /* 1 / u_kk, u_k,k+1, u_k,k+2, l_k+1,k */
+    float rd[NC], u1[NC], u2[NC], l[NC]; /* 1 / u_kk, u_k,k+1, u_k,k+2, l_k+1,k */
     unsigned piv;
 };
 
 __device__ __forceinline__ void tri_lu(TriLU &f, int n, float lambda, float tiny, const HWs &w,
                                        const Pair &g)
 {
-    float d[32], e[32];
+    float d[NC], e[NC];
 
 #pragma unroll
-    for (int k = 0; k < 32; k += 4) {
+    for (int k = 0; k < NC; k += 4) {
         const float4 a = *(const float4 *)(w.d + k), b = *(const float4 *)(w.e + k);
 
         d[k] = k < n ? a.x : 0.f;
@@ -641,9 +662,9 @@ __device__ __forceinline__ void tri_lu(TriLU &f, int n, float lambda, float tiny
 
     f.piv = 0u;
 #pragma unroll
-    for (int k = 0; k < 32; k++) {
-        const float sub = e[k], nd = k < 31 ? d[k + 1] - lambda : 0.f;
-        const float ns = k < 31 ? e[k + 1] : 0.f;
+    for (int k = 0; k < NC; k++) {
+        const float sub = e[k], nd = k < NC - 1 ? d[k + 1] - lambda : 0.f;
+        const float ns = k < NC - 1 ? e[k + 1] : 0.f;
         const bool swap = !(fabsf(dd) >= fabsf(sub));
         const float dc = fabsf(dd) < tiny ? (dd < 0.f ? -tiny : tiny) : dd;
         const float r = rcp_approx(swap ? sub : dc);
@@ -666,11 +687,11 @@ __device__ __forceinline__ void tri_lu(TriLU &f, int n, float lambda, float tiny
 
 /* Solve (tri - lambda) with the LU of tri_lu, in place on yr (every lane,
    same values). */
-__device__ __forceinline__ void tri_solve(float (&yr)[32], int n, unsigned long long piv,
+__device__ __forceinline__ void tri_solve(float (&yr)[NC], int n, unsigned long long piv,
                                           const HWs &w)
 {
 #pragma unroll
-    for (int k = 0; k < 31; k++) {
+    for (int k = 0; k < NC - 1; k++) {
         if (k >= n - 1)
             break;
         if ((piv >> k) & 1ull) {
@@ -682,7 +703,7 @@ __device__ __forceinline__ void tri_solve(float (&yr)[32], int n, unsigned long 
         yr[k + 1] -= w.lu[k].w * yr[k];
     }
 #pragma unroll
-    for (int k = 31; k >= 0; k--) {
+    for (int k = NC - 1; k >= 0; k--) {
         if (k > n - 1)
             continue;
         const float4 u = w.lu[k];
@@ -696,10 +717,10 @@ __device__ __forceinline__ void tri_solve(float (&yr)[32], int n, unsigned long 
     }
 }
 
-__device__ __forceinline__ void tri_solve(float (&yr)[32], const TriLU &f)
+__device__ __forceinline__ void tri_solve(float (&yr)[NC], const TriLU &f)
 {
 #pragma unroll
-    for (int k = 0; k < 31; k++) {
+    for (int k = 0; k < NC - 1; k++) {
         const bool swap = ((f.piv >> k) & 1u) != 0u;
         const float a = swap ? yr[k + 1] : yr[k], b = swap ? yr[k] : yr[k + 1];
 
@@ -707,12 +728,12 @@ __device__ __forceinline__ void tri_solve(float (&yr)[32], const TriLU &f)
         yr[k + 1] = fmaf(-f.l[k], a, b);
     }
 #pragma unroll
-    for (int k = 31; k >= 0; k--) {
+    for (int k = NC - 1; k >= 0; k--) {
         float v = yr[k];
 
-        if (k < 31)
+        if (k < NC - 1)
             v = fmaf(-f.u1[k], yr[k + 1], v);
-        if (k < 30)
+        if (k < NC - 2)
             v = fmaf(-f.u2[k], yr[k + 2], v);
         yr[k] = v * f.rd[k];
     }
@@ -722,7 +743,7 @@ __device__ __forceinline__ void tri_solve(float (&yr)[32], const TriLU &f)
    returns the components of rows i0, i1 in z0, z1; y (tridiagonal vector)
    is left in yr. */
 __device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g, float2 &z0,
-                           float2 &z1, float (&yr)[32], float &lambda, float &norm,
+                           float2 &z1, float (&yr)[NC], float &lambda, float &norm,
                            unsigned long long &piv)
 {
     unsigned status = 0;
@@ -735,7 +756,7 @@ __device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g
     tri_lu(f, n, lambda, tiny, w, g);
     piv = f.piv;
 #pragma unroll
-    for (int k = 0; k < 32; k++)
+    for (int k = 0; k < NC; k++)
         yr[k] = 1.f;
 #pragma unroll 1
     for (int it = 0; it < 3; it++) {
@@ -743,7 +764,7 @@ __device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g
         float nrm = 0.f, odd = 0.f;
 
 #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
+        for (int k = 0; k < NC; k += 2) {
             nrm = fmaxf(nrm, k < n ? fabsf(yr[k]) : 0.f);
             odd = fmaxf(odd, k + 1 < n ? fabsf(yr[k + 1]) : 0.f);
         }
@@ -751,21 +772,21 @@ __device__ unsigned eigvec(int n, int index, const HWs &w, int ld, const Pair &g
         const float inv = __frcp_rn(nrm);
 
 #pragma unroll
-        for (int k = 0; k < 32; k++)
+        for (int k = 0; k < NC; k++)
             yr[k] *= inv;
     }
     const int i0 = g.gl, i1 = g.gl + 16;
     float y0 = 0.f, y1 = 0.f;
 
 #pragma unroll
-    for (int k = 0; k < 32; k++) {
+    for (int k = 0; k < NC; k++) {
         if (k == i0)
             y0 = yr[k];
-        if (k == i1)
+        if (TWO && k == i1)
             y1 = yr[k];
     }
     z0 = make_float2(i0 < n ? y0 : 0.f, 0.f);
-    z1 = make_float2(i1 < n ? y1 : 0.f, 0.f);
+    z1 = make_float2(TWO && i1 < n ? y1 : 0.f, 0.f);
     /* z = H_0 .. H_{n-2} y */
     apply_q(n, ld, w, g, false, z0, z1);
     return status;
@@ -807,7 +828,7 @@ __device__ __forceinline__ double rcp_newton(double d)
    buffer that was last read before the barrier of the step before it. False
    when a pivot's magnitude is not above `floor`. */
 template <class G>
-__device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor, double *rs,
+__device__ bool sweep16(double (&g0)[NC], double (&g1)[NC], int n, double floor, double *rs,
                         const G &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
@@ -815,7 +836,8 @@ __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor,
     double *r = rs;
 
     r[i0] = g0[0];
-    r[i1] = g1[0];
+    if (TWO)
+        r[i1] = g1[0];
     gsync(g);
     /* a half that met a small pivot stays in step; its values are unused */
     bool ok = fabs(r[0]) > floor;
@@ -826,28 +848,33 @@ __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor,
         const bool piv0 = i0 == k, piv1 = i1 == k;
         /* the pivot row scales by 1 / a_kk: a_kj - (1 - 1 / a_kk) a_kj, with
            a_kj from rs (equal to the row's own value up to rounding) */
-        const double f0 = piv0 ? 1.0 - id : g0[0] * id, f1 = piv1 ? 1.0 - id : g1[0] * id;
-        double *rn = r == rs + 64 ? rs : r + 32;
+        const double f0 = piv0 ? 1.0 - id : g0[0] * id, f1 = !TWO ? 0.0 : piv1 ? 1.0 - id : g1[0] * id;
+        double *rn = r == rs + 2 * NC ? rs : r + NC;
         const double a1 = r[1];
 
         g0[0] = fma(-f0, a1, g0[1]);
-        g1[0] = fma(-f1, a1, g1[1]);
-        rn[(i0 - k - 1) & 31] = g0[0];
-        rn[(i1 - k - 1) & 31] = g1[0];
+        if (TWO)
+            g1[0] = fma(-f1, a1, g1[1]);
+        rn[(i0 - k - 1) & (NC - 1)] = g0[0];
+        if (TWO)
+            rn[(i1 - k - 1) & (NC - 1)] = g1[0];
         gsync(g);
         const double dn = rn[0], idn = rcp_newton(dn); /* unused after the last step */
 
 #pragma unroll
-        for (int q = 2; q < 32; q += 2) {
+        for (int q = 2; q < NC; q += 2) {
             const double2 a = *(const double2 *)&r[q];
 
             g0[q - 1] = fma(-f0, a.x, g0[q]);
-            g1[q - 1] = fma(-f1, a.x, g1[q]);
             g0[q] = fma(-f0, a.y, g0[q + 1]);
-            g1[q] = fma(-f1, a.y, g1[q + 1]);
+            if (TWO) {
+                g1[q - 1] = fma(-f1, a.x, g1[q]);
+                g1[q] = fma(-f1, a.y, g1[q + 1]);
+            }
         }
-        g0[31] = piv0 ? -id : f0;
-        g1[31] = piv1 ? -id : f1;
+        g0[NC - 1] = piv0 ? -id : f0;
+        if (TWO)
+            g1[NC - 1] = piv1 ? -id : f1;
         r = rn;
         id = idn;
         ok = ok && (k == n - 1 || fabs(dn) > floor);
@@ -856,21 +883,21 @@ __device__ bool sweep16(double (&g0)[32], double (&g1)[32], int n, double floor,
 }
 
 /* Rows i0, i1 of a matrix whose register column p is true column
-   (p + rot) & 31, scaled by s, into dst (n x ld). */
+   (p + rot) & (NC - 1), scaled by s, into dst (n x ld). */
 __device__ __forceinline__ void store_rows(double *dst, int ld, int n, int rot, double s,
-                                           const double (&g0)[32], const double (&g1)[32],
+                                           const double (&g0)[NC], const double (&g1)[NC],
                                            const Grp &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
 
 #pragma unroll
-    for (int p = 0; p < 32; p++) {
-        const int j = (p + rot) & 31;
+    for (int p = 0; p < NC; p++) {
+        const int j = (p + rot) & (NC - 1);
 
         if (j < n) {
             if (i0 < n)
                 dst[i0 * ld + j] = s * g0[p];
-            if (i1 < n)
+            if (TWO && i1 < n)
                 dst[i1 * ld + j] = s * g1[p];
         }
     }
@@ -878,24 +905,25 @@ __device__ __forceinline__ void store_rows(double *dst, int ld, int n, int rot, 
 
 /* (o0, o1) = rows i0, i1 of A times B; A and B n x ld (memory). */
 __device__ void rows_times(const double *A, const double *B, int ld, int n, int i0, int i1,
-                           double (&o0)[32], double (&o1)[32])
+                           double (&o0)[NC], double (&o1)[NC])
 {
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < NC; j++) {
         o0[j] = 0.0;
         o1[j] = 0.0;
     }
     for (int k = 0; k < n; k++) {
         const double *row = B + k * ld;
-        const double x0 = i0 < n ? A[i0 * ld + k] : 0.0, x1 = i1 < n ? A[i1 * ld + k] : 0.0;
+        const double x0 = i0 < n ? A[i0 * ld + k] : 0.0, x1 = TWO && i1 < n ? A[i1 * ld + k] : 0.0;
 
 #pragma unroll
-        for (int j = 0; j < 32; j++)
+        for (int j = 0; j < NC; j++)
             if (j < n) {
                 const double b = row[j];
 
                 o0[j] = fma(x0, b, o0[j]);
-                o1[j] = fma(x1, b, o1[j]);
+                if (TWO)
+                    o1[j] = fma(x1, b, o1[j]);
             }
     }
 }
@@ -1040,7 +1068,7 @@ __device__ __noinline__ unsigned emi_fallback(int n, int ld, HWs w, double *A, d
     gsync(g);
     if (squared) {
         /* (|T|^2)^-1 |T|, with the intermediate inverse in V */
-        double g0[32], g1[32];
+        double g0[NC], g1[NC];
 
         rows_times(A, A, ld, n, i0, i1, g0, g1);
         if (sweep16(g0, g1, n, 1.0e-300, w.rs, g)) {
@@ -1050,8 +1078,8 @@ __device__ __noinline__ unsigned emi_fallback(int n, int ld, HWs w, double *A, d
             gsync(g);
             rows_times(V, A, ld, n, i0, i1, g0, g1);
 #pragma unroll
-            for (int j = 0; j < 32; j++)
-                mx = fmax(mx, fmax(fabs(g0[j]), fabs(g1[j])));
+            for (int j = 0; j < NC; j++)
+                mx = fmax(mx, TWO ? fmax(fabs(g0[j]), fabs(g1[j])) : fabs(g0[j]));
             mx = gmaxd(mx, g);
             if (mx == mx && n * mx < 1.0e8) {
                 gsync(g);
@@ -1072,16 +1100,17 @@ __device__ __noinline__ unsigned emi_fallback(int n, int ld, HWs w, double *A, d
 #define TC_LOWER(i, j) ((i) > (j) ? (i) * ld + (j) : (j) * ld + (i))
 
 /* Rows i0, i1 of |T| from the slots that load_T filled. */
-__device__ __forceinline__ void load_abs(double (&g0)[32], double (&g1)[32], int ld_,
+__device__ __forceinline__ void load_abs(double (&g0)[NC], double (&g1)[NC], int ld_,
                                          const HWs &w, const Pair &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16, ld = opaque(ld_);
     const double *A = (const double *)w.T;
 
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < NC; j++) {
         g0[j] = A[j >= 16 ? j * ld + i0 : TC_LOWER(i0, j)];
-        g1[j] = A[j < 16 ? i1 * ld + j : TC_LOWER(i1, j)];
+        if (TWO)
+            g1[j] = A[j < 16 ? i1 * ld + j : TC_LOWER(i1, j)];
     }
 }
 
@@ -1102,23 +1131,25 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
 {
     const Grp g = alone(pg);
     const int i0 = g.gl, i1 = g.gl + 16;
-    double g0[32], g1[32];
+    double g0[NC], g1[NC];
     unsigned st = 0;
 
     load_abs(g0, g1, ld, w, pg);
     const bool swept = sweep16(g0, g1, n, 1.0e-5, w.rs, pg);
 
 #pragma unroll 1
-    for (int k = n; k < 32; k++) {
-        const double t0 = g0[0], t1 = g1[0];
+    for (int k = n; k < NC; k++) {
+        const double t0 = g0[0], t1 = TWO ? g1[0] : 0.0;
 
 #pragma unroll
-        for (int q = 0; q < 31; q++) {
+        for (int q = 0; q < NC - 1; q++) {
             g0[q] = g0[q + 1];
-            g1[q] = g1[q + 1];
+            if (TWO)
+                g1[q] = g1[q + 1];
         }
-        g0[31] = t0;
-        g1[31] = t1;
+        g0[NC - 1] = t0;
+        if (TWO)
+            g1[NC - 1] = t1;
     }
     /* the largest magnitude left of the diagonal, as an integer: the upper
        words first, then the lower words of those that have the largest (64
@@ -1126,17 +1157,18 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
     unsigned top = 0u, low = 0u;
 
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < NC; j++) {
         if (j < 16)
             top = max(top, (unsigned)__double2hiint(g0[j]) & 0x7fffffffu);
-        top = max(top, (unsigned)__double2hiint(g1[j]) & 0x7fffffffu);
+        if (TWO)
+            top = max(top, (unsigned)__double2hiint(g1[j]) & 0x7fffffffu);
     }
     top = gmaxu(top, pg);
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < NC; j++) {
         if (j < 16 && ((unsigned)__double2hiint(g0[j]) & 0x7fffffffu) == top)
             low = max(low, (unsigned)__double2loint(g0[j]));
-        if (((unsigned)__double2hiint(g1[j]) & 0x7fffffffu) == top)
+        if (TWO && ((unsigned)__double2hiint(g1[j]) & 0x7fffffffu) == top)
             low = max(low, (unsigned)__double2loint(g1[j]));
     }
     const double mx = __hiloint2double((int)top, (int)gmaxu(low, pg));
@@ -1152,14 +1184,15 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
         /* batches of eight columns: their loads, arithmetic, stores; the
            diagonal's T is 1 */
 #pragma unroll
-        for (int jb = 0; jb < 32; jb += 8) {
+        for (int jb = 0; jb < NC; jb += 8) {
             float2 m0[8], m1[8];
 
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 if (jb < 16)
                     m0[u] = w.T[(jb + u) * lv + i0];
-                m1[u] = w.T[(jb + u) * lv + i1];
+                if (TWO)
+                    m1[u] = w.T[(jb + u) * lv + i1];
             }
 #pragma unroll
             for (int u = 0; u < 8; u++) {
@@ -1171,10 +1204,12 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
                     m0[u] = make_float2((float)(-g0[j] * (double)m0[u].x),
                                         (float)(g0[j] * (double)m0[u].y));
                 }
-                else if (j == i1)
-                    m1[u] = make_float2(1.f, 0.f);
-                m1[u] = make_float2((float)(-g1[j] * (double)m1[u].x),
-                                    (float)(g1[j] * (double)m1[u].y));
+                if (TWO) {
+                    if (jb >= 16 && j == i1)
+                        m1[u] = make_float2(1.f, 0.f);
+                    m1[u] = make_float2((float)(-g1[j] * (double)m1[u].x),
+                                        (float)(g1[j] * (double)m1[u].y));
+                }
             }
 #pragma unroll
             for (int u = 0; u < 8; u++) {
@@ -1185,14 +1220,14 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
                     w.T[i0 * lv + j] = m0[u];
                     gj[i0] = -g0[j];
                 }
-                if (j <= e1) {
+                if (TWO && j <= e1) {
                     w.T[i1 * lv + j] = m1[u];
                     gj[i1] = -g1[j];
                 }
             }
         }
     }
-    if (!ok) {
+    auto fall_back = [&]() {
         st |= emi_fallback<ADJ>(n, ld, w, A, V, lam, g, !swept);
         for (int r = g.gl; r < n; r += 16)
             for (int j = 0; j <= r; j++) {
@@ -1203,7 +1238,18 @@ __device__ unsigned emi_matrix(int n, int ld, const HWs &w, double *A, double *V
                     make_float2((float)(a * (double)t.x), -(float)(a * (double)t.y));
                 w.G[tc_pidx(n, j, r)] = a;
             }
+    };
+
+    if (TWO) {
+        if (!ok)
+            fall_back();
     }
+    else if (__any_sync(FULL, !ok))
+        for (int h = 0; h < 32; h += 16) {
+            if (!ok && g.base == h)
+                fall_back();
+            gsync(pg);
+        }
     gsync(pg);
     return st;
 }
@@ -1225,7 +1271,7 @@ __device__ __forceinline__ double2 mval(const HWs &w, int ld, int i, int j)
    parts solved with the LU, the y component removed again, and the result
    mapped back by Q. Scratch: the first 32 float2 of w.x. */
 template <class G>
-__device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (&yr)[32],
+__device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (&yr)[NC],
                           unsigned long long piv, float2 b0, float2 b1, float2 &t0, float2 &t1)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
@@ -1237,13 +1283,14 @@ __device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (
     float2 *bs = (float2 *)w.x;
 
     bs[i0] = b0;
-    bs[i1] = b1;
+    if (TWO)
+        bs[i1] = b1;
     gsync(g);
-    float tr_[32], ti_[32];
+    float tr_[NC], ti_[NC];
     float ynrm = 0.f, cr = 0.f, ci = 0.f;
 
 #pragma unroll
-    for (int k = 0; k < 32; k++) {
+    for (int k = 0; k < NC; k++) {
         const float2 bk = k < n ? bs[k] : make_float2(0.f, 0.f);
 
         ynrm = fmaf(yr[k], yr[k], ynrm);
@@ -1256,21 +1303,21 @@ __device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (
     cr /= ynrm;
     ci /= ynrm;
 #pragma unroll
-    for (int k = 0; k < 32; k++) {
+    for (int k = 0; k < NC; k++) {
         tr_[k] = fmaf(-cr, yr[k], tr_[k]);
         ti_[k] = fmaf(-ci, yr[k], ti_[k]);
     }
     /* one solve per lane: the real parts in lanes 0-7, the imaginary parts
        in lanes 8-15, exchanged afterwards */
     {
-        float v[32];
+        float v[NC];
 
 #pragma unroll
-        for (int k = 0; k < 32; k++)
+        for (int k = 0; k < NC; k++)
             v[k] = g.gl >= 8 ? ti_[k] : tr_[k];
         tri_solve(v, n, piv, w);
 #pragma unroll
-        for (int k = 0; k < 32; k++) {
+        for (int k = 0; k < NC; k++) {
             tr_[k] = __shfl_sync(g.members(), v[k], g.base);
             ti_[k] = __shfl_sync(g.members(), v[k], g.base | 8);
         }
@@ -1278,7 +1325,7 @@ __device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (
     float dr = 0.f, di = 0.f;
 
 #pragma unroll
-    for (int k = 0; k < 32; k++)
+    for (int k = 0; k < NC; k++)
         if (k < n) {
             dr = fmaf(yr[k], tr_[k], dr);
             di = fmaf(yr[k], ti_[k], di);
@@ -1288,10 +1335,10 @@ __device__ void solve_off(int n, int ld, const HWs &w, const G &g, const float (
     t0 = make_float2(0.f, 0.f);
     t1 = t0;
 #pragma unroll
-    for (int k = 0; k < 32; k++) {
+    for (int k = 0; k < NC; k++) {
         if (k == i0 && k < n)
             t0 = make_float2(fmaf(-dr, yr[k], tr_[k]), fmaf(-di, yr[k], ti_[k]));
-        if (k == i1 && k < n)
+        if (TWO && k == i1 && k < n)
             t1 = make_float2(fmaf(-dr, yr[k], tr_[k]), fmaf(-di, yr[k], ti_[k]));
     }
     /* t = Q t = H_0 .. H_{n-2} t */
@@ -1321,7 +1368,8 @@ __device__ __noinline__ double4 refine(int n, int ld, HWs w, Grp g, double2 x0, 
     x1.x *= inrm;
     x1.y *= inrm;
     w.x[i0] = x0;
-    w.x[i1] = x1;
+    if (TWO)
+        w.x[i1] = x1;
     gsync(g);
     /* u = M x (rows i0, i1), mu = x^H u */
     double2 u0 = make_double2(0.0, 0.0), u1 = u0;
@@ -1335,7 +1383,7 @@ __device__ __noinline__ double4 refine(int n, int ld, HWs w, Grp g, double2 x0, 
             u0.x += m.x * xj.x - m.y * xj.y;
             u0.y += m.x * xj.y + m.y * xj.x;
         }
-        if (i1 < n) {
+        if (TWO && i1 < n) {
             const double2 m = mval(w, ld, i1, j);
 
             u1.x += m.x * xj.x - m.y * xj.y;
@@ -1351,7 +1399,7 @@ __device__ __noinline__ double4 refine(int n, int ld, HWs w, Grp g, double2 x0, 
 
     if (i0 >= n)
         r0 = make_double2(0.0, 0.0);
-    if (i1 >= n)
+    if (!TWO || i1 >= n)
         r1 = make_double2(0.0, 0.0);
     const double rmax = gmaxd(fmax(fmax(fabs(r0.x), fabs(r0.y)), fmax(fabs(r1.x), fabs(r1.y))), g);
 
@@ -1360,10 +1408,10 @@ __device__ __noinline__ double4 refine(int n, int ld, HWs w, Grp g, double2 x0, 
         return make_double4(x0.x, x0.y, x1.x, x1.y);
     const double sc = 1.0 / rmax;
     float2 t0, t1;
-    float yr[32];
+    float yr[NC];
 
 #pragma unroll
-    for (int k = 0; k < 32; k++)
+    for (int k = 0; k < NC; k++)
         yr[k] = w.y[k];
 
     solve_off(n, ld, w, g, yr, piv, make_float2((float)(r0.x * sc), (float)(r0.y * sc)),
@@ -1470,7 +1518,7 @@ __device__ __forceinline__ void t_first(TFirst &f, int n, int p, bool inrange,
     const float2 *sums = gram + tc_gram_at(npu, inrange ? p : 0, 0);
 
     f.d0 = (inrange && i0 < n) ? sums[tc_pidx(n, i0, i0)].x : 1.f;
-    f.d1 = (inrange && i1 < n) ? sums[tc_pidx(n, i1, i1)].x : 1.f;
+    f.d1 = (TWO && inrange && i1 < n) ? sums[tc_pidx(n, i1, i1)].x : 1.f;
     gram_batch(f.a, 0, npu, inrange, sums, g);
     gram_batch(f.b, LT_BATCH, npu, inrange, sums, g);
 }
@@ -1494,7 +1542,7 @@ __device__ void load_T(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
 
     if (i0 < n)
         w.nrm[i0] = d0 > 0.f ? __frcp_rn(__fsqrt_rn(d0)) : 0.f;
-    if (i1 < n)
+    if (TWO && i1 < n)
         w.nrm[i1] = d1 > 0.f ? __frcp_rn(__fsqrt_rn(d1)) : 0.f;
     gsync(g);
     const float fl = (float)looks;
@@ -1537,7 +1585,7 @@ __device__ bool linked16(int n, int ld, const float2 *T, const Pair &g)
     while (__any_sync(FULL, todo != 0u && reached != all)) {
         const int f = todo ? __ffs(todo) - 1 : 0;
         const float2 a = i0 < n ? T[min(i0, f) * ld + max(i0, f)] : make_float2(0.f, 0.f);
-        const float2 b = i1 < n ? T[min(i1, f) * ld + max(i1, f)] : make_float2(0.f, 0.f);
+        const float2 b = TWO && i1 < n ? T[min(i1, f) * ld + max(i1, f)] : make_float2(0.f, 0.f);
         const unsigned lo = __ballot_sync(FULL, a.x != 0.f || a.y != 0.f) >> g.base;
         const unsigned hi = __ballot_sync(FULL, b.x != 0.f || b.y != 0.f) >> g.base;
         const unsigned nw = ((lo & 0xFFFFu) | (hi << 16)) & ~reached;
@@ -1559,17 +1607,17 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Pair &g, double2 z0d
     const float2 z0 = make_float2((float)z0d.x, (float)z0d.y);
     const float2 z1 = make_float2((float)z1d.x, (float)z1d.y);
     const int i0 = g.gl, i1 = g.gl + 16;
-    const float m0 = i0 < n ? hypotf(z0.x, z0.y) : 0.f, m1 = i1 < n ? hypotf(z1.x, z1.y) : 0.f;
+    const float m0 = i0 < n ? hypotf(z0.x, z0.y) : 0.f, m1 = TWO && i1 < n ? hypotf(z1.x, z1.y) : 0.f;
     const float mx = gmaxf(fmaxf(m0, m1), g);
     int ref = n / 2;
-    const float mref = gbcast(ref < 16 ? m0 : m1, ref, g);
+    const float mref = gbcast(!TWO || ref < 16 ? m0 : m1, ref, g);
 
     if (__any_sync(FULL, mref <= 1.0e-3f * mx)) {
         int last = -1;
 
         if (i0 < n && m0 == mx)
             last = i0;
-        if (i1 < n && m1 == mx)
+        if (TWO && i1 < n && m1 == mx)
             last = i1;
 #pragma unroll
         for (int o = 8; o; o >>= 1)
@@ -1577,14 +1625,14 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Pair &g, double2 z0d
         if (mref <= 1.0e-3f * mx)
             ref = last;
     }
-    const float zrx = gbcast(ref < 16 ? z0.x : z1.x, ref, g);
-    const float zry = gbcast(ref < 16 ? z0.y : z1.y, ref, g);
+    const float zrx = gbcast(!TWO || ref < 16 ? z0.x : z1.x, ref, g);
+    const float zry = gbcast(!TWO || ref < 16 ? z0.y : z1.y, ref, g);
     const float refm = hypotf(zrx, zry);
     const float refr = zrx / refm, refi = -zry / refm;
     const float floor_ = mx * 1.0e-3f;
 
 #pragma unroll
-    for (int t = 0; t < 2; t++) {
+    for (int t = 0; t < 1 + TWO; t++) {
         const int r = t ? i1 : i0;
         const float2 z = t ? z1 : z0;
 
@@ -1654,6 +1702,7 @@ __device__ __forceinline__ float2 t_full(const HWs &w, int ld, int i, int j)
     return i < j ? t : make_float2(t.x, -t.y);
 }
 
+#if TC_LINK_COLS == 32
 /* Gradient of gamma with respect to the pixel's coherence sums, written as
    the Hermitian matrix G (upper triangle, gbar[pidx][p]) such that
    d gamma = Re sum_ij conj(G_ij) dC_ij. The chain, in reverse:
@@ -1972,11 +2021,20 @@ __device__ void backward16(int n, int ld, const HWs &w, const Pair &g, double2 z
     }
     gsync(g);
 }
+#endif
+
+/* Warps per CTA (one CTA per SM): by the registers that the stages need (255 of
+   them for EMI's two rows of doubles, 168 for EVD; with one row per lane 128 and
+   80). */
+constexpr int half_warps(bool emi, bool adj)
+{
+    return TWO ? (emi || adj ? 8 : 12) : (emi ? 16 : 24);
+}
 
 /* ADJ: after gamma, backward16 writes the gradient of gamma with respect
    to the pixel's coherence sums into gbar (same layout as gram). */
 template <bool EMI, bool ADJ>
-__global__ void __launch_bounds__(EMI || ADJ ? 256 : 384)
+__global__ void __launch_bounds__(32 * half_warps(EMI, ADJ))
 tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                     const float2 *__restrict__ gram, const int *__restrict__ count,
                     const unsigned short *__restrict__ upper_tab,
@@ -1994,7 +2052,10 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
     const HWs w = hws(smem + (size_t)grp * L.per_group, L);
     const int n = s.n, ld = L.ld;
     const long long plane = (long long)s.rows * s.cols;
-    double *V = scratch + ((size_t)blockIdx.x * wpb * 2 + grp) * (size_t)(2 * n * ld + 32);
+    /* EMI's fallback tiers: a slot per group, or (one row per lane, more warps)
+       per warp, its halves in turn; 16 per CTA either way */
+    double *V = scratch + (TWO ? (size_t)blockIdx.x * wpb * 2 + grp
+                               : (size_t)blockIdx.x * wpb + warp) * (size_t)(2 * n * ld + 32);
     const int i0 = g.gl, i1 = g.gl + 16;
     /* the packed-entry table, read in every stage, from shared memory */
     unsigned short *s_upper = (unsigned short *)(smem + (size_t)wpb * 2 * L.per_group);
@@ -2004,7 +2065,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
     __syncthreads();
 
     if (EMI) {
-        for (int e = n * ld + g.gl; e < 32 * ld + 32; e += 16)
+        for (int e = n * ld + g.gl; e < NC * ld + 32; e += 16)
             w.T[e] = make_float2(0.f, 0.f);
         __syncthreads();
     }
@@ -2102,9 +2163,9 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
         }
         __syncthreads();
 
-        float2 r0[32], r1[32];
+        float2 r0[NC], r1[NC];
         double2 z0 = make_double2(0.0, 0.0), z1 = z0;
-        float yr[32], lambda = 0.f, norm = 0.f;
+        float yr[NC], lambda = 0.f, norm = 0.f;
         double inv_max = INFINITY;
         float2 f0 = make_float2(0.f, 0.f), f1 = f0;
         unsigned long long piv = 0ull;
@@ -2113,9 +2174,10 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
             /* stage 2: Householder reduction of T */
             if (run) {
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
+                for (int j = 0; j < NC; j++) {
                     r0[j] = (i0 < n && j < n) ? w.T[i0 * ld + j] : make_float2(0.f, 0.f);
-                    r1[j] = (i1 < n && j < n) ? w.T[i1 * ld + j] : make_float2(0.f, 0.f);
+                    if (TWO)
+                        r1[j] = (i1 < n && j < n) ? w.T[i1 * ld + j] : make_float2(0.f, 0.f);
                 }
                 gsync(g);
                 householder(r0, r1, n, w, ld, g);
@@ -2139,13 +2201,16 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                 const int ld = opaque(L.ld);
 
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
+                for (int j = 0; j < NC; j++) {
                     /* M_ij left of the diagonal, conj(M_ji) right of it */
                     const float2 a = w.T[j >= 16 ? j * ld + i0 : TC_LOWER(i0, j)];
-                    const float2 b = w.T[j < 16 ? i1 * ld + j : TC_LOWER(i1, j)];
 
                     r0[j] = make_float2(a.x, j < 16 && i0 >= j ? a.y : -a.y);
-                    r1[j] = make_float2(b.x, j < 16 || i1 >= j ? b.y : -b.y);
+                    if (TWO) {
+                        const float2 b = w.T[j < 16 ? i1 * ld + j : TC_LOWER(i1, j)];
+
+                        r1[j] = make_float2(b.x, j < 16 || i1 >= j ? b.y : -b.y);
+                    }
                 }
                 gsync(g);
                 /* The reduction parks its vectors in T's lower triangle. */
@@ -2171,7 +2236,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                 if (active && sturm16(w.d, w.e2f, n, lambda + TC_REFINE_GAP * norm,
                                       1.0e-30f + 1.0e-14f * norm) >= 2) {
 #pragma unroll
-                    for (int k = 0; k < 32; k += 4)
+                    for (int k = 0; k < NC; k += 4)
                         *(float4 *)(w.y + k) =
                             make_float4(yr[k], yr[k + 1], yr[k + 2], yr[k + 3]);
                     const double4 z = refine(n, ld, w, alone(g), z0, z1, piv);
@@ -2222,7 +2287,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
                     coh[out] = gamma;
                 if (phases)
 #pragma unroll
-                    for (int t = 0; t < 2; t++) {
+                    for (int t = 0; t < 1 + TWO; t++) {
                         const int r = t ? i1 : i0;
 
                         if (r < n) {
@@ -2236,6 +2301,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
             }
         }
         if (ADJ && q < nq) {
+#if TC_LINK_COLS == 32
             if (run)
                 backward16<EMI>(n, ld, w, g, z0, z1, ssum, yr, piv, looks, k.bias != 0, active,
                                 (double *)(smem + (size_t)grp * L.per_group + L.off_Db), gbar,
@@ -2243,6 +2309,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
             else
                 for (int t = g.gl; t < tc_npu(n); t += 16)
                     gbar[(long long)t * c.npix + p] = make_float2(0.f, 0.f);
+#endif
         }
         if (ADJ)
             prefetch_next();
@@ -2263,8 +2330,8 @@ HalfLayout half_layout(int n, int emi, int adj = 0)
 
     L.n = n;
     L.ld = n | 1;
-    /* EMI: rows from n to 31 stay zero; column indices up to 31 */
-    L.off_T = take(8 * (emi ? 32 * L.ld + 32 : n * L.ld));
+    /* EMI: rows from n to NC - 1 stay zero; column indices up to 31 */
+    L.off_T = take(8 * (emi ? NC * L.ld + 32 : n * L.ld));
     L.off_G = take(emi ? 8 * tc_npu(n) : 0);
     /* stage-local: the reciprocal date norms (T), the sweep's pivot rows
        (inverse), the Householder vectors (reduction), the solves' and the
@@ -2273,7 +2340,7 @@ HalfLayout half_layout(int n, int emi, int adj = 0)
     L.off_vw = take(16 * 64);
     L.off_rs = L.off_vw;
     L.off_x = L.off_vw;
-    L.off_lu = take(16 * 32);
+    L.off_lu = take(16 * NC);
     L.off_tau = take(8 * 32);
     L.off_d = take(4 * 32);
     L.off_e = take(4 * 32);
@@ -2292,6 +2359,7 @@ HalfLayout half_layout(int n, int emi, int adj = 0)
 
 } // namespace
 
+#if TC_LINK_COLS == 32
 size_t tc_link_half_scratch_bytes(int n, int sms)
 {
     /* EMI only, per group (two per warp, at most 8 warps per CTA, one CTA
@@ -2301,6 +2369,7 @@ size_t tc_link_half_scratch_bytes(int n, int sms)
         return 256;
     return (size_t)sms * 16 * (2 * n * (n | 1) + 32) * sizeof(double);
 }
+#endif
 
 template <bool EMI, bool ADJ>
 static cudaError_t launch_half(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
@@ -2314,11 +2383,17 @@ static cudaError_t launch_half(const TcStrip &s, const TcChunk &c, const TcLinkC
     const HalfLayout L = half_layout(s.n, EMI, ADJ);
     const size_t per_warp = 2 * (size_t)L.per_group;
     const size_t tab = ((size_t)tc_npu(s.n) * 2 + 15) & ~(size_t)15;
-    const int max_warps = EMI || ADJ ? 8 : 12;
+    const int max_warps = half_warps(EMI, ADJ);
     int wpb = (int)((227 * 1024 - tab) / per_warp);
 
     if (wpb > max_warps)
         wpb = max_warps;
+    /* few pixels: over all SMs rather than in full CTAs on some (a 48 x 40 crop
+       at 10 dates: 33 -> 21 us) */
+    const int spread = ((c.npix + 1) / 2 + sms - 1) / sms;
+
+    if (wpb > spread)
+        wpb = spread;
     if (wpb < 1)
         return cudaErrorInvalidConfiguration;
     const size_t smem = per_warp * wpb + tab;
@@ -2335,13 +2410,27 @@ static cudaError_t launch_half(const TcStrip &s, const TcChunk &c, const TcLinkC
     return cudaGetLastError();
 }
 
-cudaError_t tc_launch_link_half(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
-                                const float2 *gram, const uint32_t *mask, const int *count,
-                                const unsigned short *upper_tab, const unsigned short *pair_tab,
-                                double *scratch, float *coh, float *pairs, float *phases,
-                                unsigned char *status, int *queue, int qstride, int sms,
-                                cudaStream_t st)
+#if TC_LINK_COLS == 16
+#define TC_LAUNCH tc_launch_link_half16
+#else
+#define TC_LAUNCH tc_launch_link_half
+#endif
+
+cudaError_t TC_LAUNCH(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
+                      const float2 *gram, const uint32_t *mask, const int *count,
+                      const unsigned short *upper_tab, const unsigned short *pair_tab,
+                      double *scratch, float *coh, float *pairs, float *phases,
+                      unsigned char *status, int *queue, int qstride, int sms,
+                      cudaStream_t st)
 {
+#if TC_LINK_COLS == 32
+    /* One row per lane while the dates fit: under half the registers, twice the
+       warps, none of the second row's zeros (link stage 1.75 -> 0.99 ms for EVD
+       of 512 x 512 pixels at 10 dates; the results are the same bits). */
+    if (s.n <= 16)
+        return tc_launch_link_half16(s, c, k, gram, mask, count, upper_tab, pair_tab, scratch,
+                                     coh, pairs, phases, status, queue, qstride, sms, st);
+#endif
     if (k.emi)
         return launch_half<true, false>(s, c, k, gram, count, upper_tab, pair_tab, scratch, coh,
                                         pairs, phases, status, nullptr, mask, queue, qstride,
@@ -2351,6 +2440,7 @@ cudaError_t tc_launch_link_half(const TcStrip &s, const TcChunk &c, const TcLink
                                      st);
 }
 
+#if TC_LINK_COLS == 32
 cudaError_t tc_launch_link_adjoint(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
                                    const float2 *gram, const int *count,
                                    const unsigned short *upper_tab,
@@ -2366,3 +2456,4 @@ cudaError_t tc_launch_link_adjoint(const TcStrip &s, const TcChunk &c, const TcL
     return launch_half<false, true>(s, c, k, gram, count, upper_tab, pair_tab, scratch, coh,
                                     pairs, nullptr, nullptr, gbar, nullptr, nullptr, 0, sms, st);
 }
+#endif

@@ -933,6 +933,9 @@ cudaError_t tc_launch_link_wide(const TcStrip &s, const TcChunk &c, const TcLink
 
     if (pixels > WD_PIXELS)
         pixels = WD_PIXELS;
+    /* few pixels: over all SMs rather than in full CTAs on some */
+    if (pixels > (c.npix + sms - 1) / sms)
+        pixels = (c.npix + sms - 1) / sms;
     const size_t smem = (size_t)pixels * L.per_pixel + tab;
     const int want = (c.npix + pixels - 1) / pixels;
     const int blocks = want < sms ? want : sms;

@@ -294,6 +294,12 @@ cudaError_t tc_launch_link_half(const TcStrip &s, const TcChunk &c, const TcLink
                                 double *scratch, float *coh, float *pairs, float *phases,
                                 unsigned char *status, int *queue, int qstride, int sms,
                                 cudaStream_t st);
+cudaError_t tc_launch_link_half16(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
+                                  const float2 *gram, const uint32_t *mask, const int *count,
+                                  const unsigned short *upper_tab, const unsigned short *pair_tab,
+                                  double *scratch, float *coh, float *pairs, float *phases,
+                                  unsigned char *status, int *queue, int qstride, int sms,
+                                  cudaStream_t st);
 cudaError_t tc_launch_link_wide(const TcStrip &s, const TcChunk &c, const TcLinkConst &k,
                                 const float2 *gram, const uint32_t *mask, const int *count,
                                 const unsigned short *upper_tab, const unsigned short *pair_tab,
