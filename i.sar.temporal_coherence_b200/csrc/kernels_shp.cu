@@ -322,11 +322,27 @@ cudaError_t tc_launch_shp(const TcStrip &s, const TcChunk &c, const TcShpConst &
    homogeneous sets q's bit for p too, by an atomic OR, after a second,
    reversed walk if the series share a value. */
 
+/* x / d by a multiplication with magic = ceil(2^32 / d): the product's upper
+   word is the quotient or, beyond x d = 2^32, one more. */
+__device__ __forceinline__ int div_magic(int x, int d, unsigned magic)
+{
+    if (d == 1)
+        return x;
+    const int q = (int)__umulhi((unsigned)x, magic);
+
+    return q - (q * d > x);
+}
+
+__host__ __device__ inline unsigned magic_of(int d)
+{
+    return d > 1 ? (unsigned)((0x100000000ull + d - 1) / d) : 0u;
+}
+
 /* Word w of the mask of output pixel (y, x) of the block. */
 __device__ __forceinline__ long long blk_mask_at(const TcStrip &s, const TcShpBlock &b, int y,
                                                  int x, int w)
 {
-    const int j = (y - b.row0) / b.crows;
+    const int j = div_magic(y - b.row0, b.crows, b.crows_magic);
     const int r0 = b.row0 + j * b.crows;
     const int nr = min(b.crows, s.rows - r0);
     const int yl = y - r0;
@@ -338,12 +354,11 @@ __device__ __forceinline__ long long blk_mask_at(const TcStrip &s, const TcShpBl
     return j * b.chunk_words + w * npix + pl;
 }
 
-/* KS (TEST 0) or AD (TEST 1) of the centre series a_s against the lane's
-   candidate column bl (stride 32), both ending in an INFINITY sentinel:
-   the merge walk of tc_shp_kernel. REV: the candidate is the centre (it
-   goes first on ties, and AD counts its values). tie: the two series met
-   with equal heads. */
-template <int TEST, bool REV>
+/* AD of the centre series a_s against the lane's candidate column bl (stride
+   32), both ending in an INFINITY sentinel: the merge walk of tc_shp_kernel. REV:
+   the candidate is the centre (it goes first on ties, and its values are
+   counted). tie: the two series met with equal heads. */
+template <bool REV>
 __device__ __forceinline__ bool shp_walk(const float *a_s, const float *bl, int n,
                                          const float *tab, const TcShpConst &k, bool &tie)
 {
@@ -351,25 +366,6 @@ __device__ __forceinline__ bool shp_walk(const float *a_s, const float *bl, int 
     float av = a_s[0], bv = bl[0];
     bool eq = false;
 
-    if (TEST == 0) {
-        int d = 0;
-
-#pragma unroll 4
-        for (int j = 1; j < 2 * n; j++) {
-            const bool ta = REV ? av < bv : av <= bv;
-
-            eq |= av == bv;
-            ia += ta;
-            ib += !ta;
-            const float v = *(ta ? a_s + ia : bl + ib * 32);
-
-            av = ta ? v : av;
-            bv = ta ? bv : v;
-            d = max(d, abs(ia - ib));
-        }
-        tie = eq;
-        return d <= k.ks_max;
-    }
     float acc = 0.f;
     const float *tj = tab;
 
@@ -448,7 +444,7 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
             bool need = false;
 
             if (c < s.area) {
-                const int dy = c / s.wr, dx = c - dy * s.wr;
+                const int dy = div_magic(c, s.wr, b.wr_magic), dx = c - dy * s.wr;
 
                 if (valid[(long long)(y + dy) * s.W + x + dx]) {
                     const int yq = y + dy - s.wa / 2, xq = x + dx - s.wr / 2;
@@ -470,7 +466,7 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
             const int e = r0 + lane;
             const bool act = e < cnt;
             const int c = act ? list[e] : 0;
-            const int dy = c / s.wr, dx = c - dy * s.wr;
+            const int dy = div_magic(c, s.wr, b.wr_magic), dx = c - dy * s.wr;
             const long long q = (long long)(y + dy) * s.W + x + dx;
             bool ok = false, tie = false;
 
@@ -506,7 +502,7 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
                         for (int j = 0; j < n; j++)
                             b_s[j * 32 + lane] = bq[j];
                     b_s[n * 32 + lane] = INFINITY;
-                    ok = shp_walk<TEST == 2 ? 0 : TEST, false>(a_s, b_s + lane, n, tab, k, tie);
+                    ok = shp_walk<false>(a_s, b_s + lane, n, tab, k, tie);
                 }
             }
             /* this pixel's bits, gathered into lane w for word w */
@@ -530,7 +526,7 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
                     if (TEST != 2 && tie) {
                         bool t2;
 
-                        okr = shp_walk<TEST == 2 ? 0 : TEST, true>(a_s, b_s + lane, n, tab, k, t2);
+                        okr = shp_walk<true>(a_s, b_s + lane, n, tab, k, t2);
                     }
                     if (okr) {
                         const int cr = s.area - 1 - c;
@@ -545,6 +541,162 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
             atomicOr(&mask[blk_mask_at(s, b, y, x, lane)], own);
         __syncwarp();
     }
+}
+
+/* KS without the merge walk. With both series sorted, the walk's largest
+   |ia - ib| stays within m = ks_max exactly when (centre a first on ties)
+       b[i - m] < a[i]  and  a[i - m] <= b[i]   for all i >= m:
+   after taking a[i] the walk holds i + 1 values of a and the b's below a[i], and
+   after taking b[i] i + 1 of b and the a's not above it. Comparisons at fixed
+   places: the candidate's series streams past two copies of the centre's,
+   shifted by m either way and padded with NaN, whose comparisons all fail; the
+   decision with the candidate as the centre (the same with < and <= exchanged)
+   comes from the same values, so ties need no second pass.
+
+   One warp per output pixel as in tc_shp_pair_kernel. The 32 candidates' series
+   come in by coalesced loads (a window row's pixels are contiguous) into rows of
+   an odd length, one row per lane. About 5 instructions per value against the
+   walk's 10 per step and two steps per value, bound by instruction issue as that
+   was: SHP stage 1.37 -> 0.86 ms on 250 x 1000 pixels at 30 dates, 2.33 -> 1.37
+   ms on 96 x 2048 at 60, 0.69 -> 0.54 ms on 512 x 512 at 10 (there the lists of
+   candidates and the bits set for the other pixel weigh as much). */
+__global__ void __launch_bounds__(256)
+tc_shp_ks_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restrict__ amp,
+                 const unsigned char *__restrict__ valid, uint32_t *__restrict__ mask, int pair)
+{
+    extern __shared__ float4 sm4[];
+    const int n = s.n, n4 = (n + 3) & ~3, ld = n | 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wpb = blockDim.x >> 5;
+    /* floats per warp, a multiple of 4: see tc_ks_floats */
+    const int per_warp = 2 * n4 + ((32 * ld + 4 + 32 + (s.area + 1) / 2 + 3) & ~3);
+    float *lo = (float *)sm4 + warp * per_warp; /* a[j - m] */
+    float *hi = lo + n4;                        /* a[j + m] */
+    float *stage = hi + n4;                     /* 32 rows of ld, 4 to spare */
+    int *rel = (int *)(stage + 32 * ld + 4);    /* the candidates' places */
+    unsigned short *list = (unsigned short *)(rel + 32);
+    const int cc = (s.wa / 2) * s.wr + s.wr / 2; /* the centre's own index */
+    const long long npx = (long long)b.nrows * s.cols;
+    const int m = k.ks_max;
+    /* elements of the staging loop: single values, or pairs where every series
+       starts on 8 bytes */
+    const int nu = pair ? n / 2 : n;
+    const unsigned magic = magic_of(nu);
+
+    for (long long pix = blockIdx.x * (long long)wpb + warp; pix < npx;
+         pix += (long long)gridDim.x * wpb) {
+        const int y = b.row0 + (int)(pix / s.cols), x = (int)(pix % s.cols);
+        const long long centre = (long long)(y + s.wa / 2) * s.W + x + s.wr / 2;
+        const float *base = amp + ((long long)y * s.W + x) * n;
+
+        if (!valid[centre])
+            continue;
+        for (int j = lane; j < n4; j += 32) {
+            lo[j] = j >= m && j < n ? amp[centre * n + j - m] : __int_as_float(0x7fffffff);
+            hi[j] = j < n - m ? amp[centre * n + j + m] : __int_as_float(0x7fffffff);
+        }
+        int cnt = 0;
+
+        for (int w = 0; w < s.mask_words; w++) {
+            const int c = w * 32 + lane;
+            bool need = false;
+
+            if (c < s.area) {
+                const int dy = div_magic(c, s.wr, b.wr_magic), dx = c - dy * s.wr;
+
+                if (valid[(long long)(y + dy) * s.W + x + dx]) {
+                    const int yq = y + dy - s.wa / 2, xq = x + dx - s.wr / 2;
+
+                    need = c >= cc ||
+                           !(yq >= b.row0 && yq < b.row0 + b.nrows && xq >= 0 && xq < s.cols);
+                }
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, need);
+
+            if (need)
+                list[cnt + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)c;
+            cnt += __popc(bal);
+        }
+        __syncwarp();
+        uint32_t own = 0u; /* lane w: word w of this pixel's bits */
+
+        for (int r0 = 0; r0 < cnt; r0 += 32) {
+            const int e = r0 + lane;
+            const bool act = e < cnt;
+            const int c = act ? list[e] : 0;
+            const int dy = div_magic(c, s.wr, b.wr_magic), dx = c - dy * s.wr;
+
+            /* an idle lane's row: candidate 0's, inside the strip */
+            rel[lane] = (dy * s.W + dx) * n;
+            __syncwarp();
+            if (pair) {
+#pragma unroll 5
+                for (int u = lane; u < 32 * nu; u += 32) {
+                    const int q = div_magic(u, nu, magic), j = 2 * (u - q * nu);
+                    const float2 v = *(const float2 *)(base + rel[q] + j);
+
+                    stage[q * ld + j] = v.x;
+                    stage[q * ld + j + 1] = v.y;
+                }
+            }
+            else {
+#pragma unroll 5
+                for (int u = lane; u < 32 * nu; u += 32) {
+                    const int q = div_magic(u, nu, magic), j = u - q * nu;
+
+                    stage[q * ld + j] = base[rel[q] + j];
+                }
+            }
+            __syncwarp();
+            const float *row = stage + lane * ld;
+            bool fwd = act, rev = act;
+
+            /* places from n on: NaN against whatever follows the row */
+#pragma unroll 2
+            for (int j = 0; j < n; j += 4) {
+                const float4 l = *(const float4 *)(lo + j), h = *(const float4 *)(hi + j);
+                const float v0 = row[j], v1 = row[j + 1], v2 = row[j + 2], v3 = row[j + 3];
+
+                fwd &= !(v0 >= h.x) & !(l.x > v0) & !(v1 >= h.y) & !(l.y > v1);
+                rev &= !(v0 > h.x) & !(l.x >= v0) & !(v1 > h.y) & !(l.y >= v1);
+                fwd &= !(v2 >= h.z) & !(l.z > v2) & !(v3 >= h.w) & !(l.w > v3);
+                rev &= !(v2 > h.z) & !(l.z >= v2) & !(v3 > h.w) & !(l.w >= v3);
+            }
+            /* this pixel's bits, gathered into lane w for word w */
+            const int wlo = list[r0] >> 5, whi = list[min(r0 + 31, cnt - 1)] >> 5;
+
+            for (int w = wlo; w <= whi; w++) {
+                const unsigned v =
+                    __reduce_or_sync(0xffffffffu, fwd && (c >> 5) == w ? 1u << (c & 31) : 0u);
+
+                if (lane == w)
+                    own |= v;
+            }
+            /* q's bit for this pixel, when q is an output pixel of the
+               block that does not test the pair itself */
+            if (rev && c > cc) {
+                const int yq = y + dy - s.wa / 2, xq = x + dx - s.wr / 2;
+
+                if (yq < b.row0 + b.nrows && xq >= 0 && xq < s.cols) {
+                    const int cr = s.area - 1 - c;
+
+                    atomicOr(&mask[blk_mask_at(s, b, yq, xq, cr >> 5)], 1u << (cr & 31));
+                }
+            }
+            __syncwarp();
+        }
+        if (lane < s.mask_words && own)
+            atomicOr(&mask[blk_mask_at(s, b, y, x, lane)], own);
+        __syncwarp();
+    }
+}
+
+/* Shared floats per warp of tc_shp_ks_kernel. */
+static int tc_ks_floats(int n, int area)
+{
+    const int n4 = (n + 3) & ~3;
+
+    return 2 * n4 + ((32 * (n | 1) + 4 + 32 + (area + 1) / 2 + 3) & ~3);
 }
 
 /* SHP counts of the block's output pixels from their masks; -1 for an
@@ -568,11 +720,15 @@ __global__ void tc_shp_count_kernel(TcStrip s, TcShpBlock b, const unsigned char
     }
 }
 
-cudaError_t tc_launch_shp_block(const TcStrip &s, const TcShpBlock &b, const TcShpConst &k,
+cudaError_t tc_launch_shp_block(const TcStrip &s, const TcShpBlock &blk, const TcShpConst &k,
                                 const float *amp, const unsigned char *valid,
                                 const float2 *logstat, uint32_t *mask, int *count, int sms,
                                 cudaStream_t st)
 {
+    TcShpBlock b = blk;
+
+    b.wr_magic = magic_of(s.wr);
+    b.crows_magic = magic_of(b.crows);
     const int threads = 256, wpb = threads / 32;
     const int tab = k.test == 1 ? (s.n + 1) * (2 * s.n - 1) : 0;
     const int per_warp = (s.n + 1) + (s.n + 1) * 32 + (s.area + 1) / 2;
@@ -587,13 +743,15 @@ cudaError_t tc_launch_shp_block(const TcStrip &s, const TcShpBlock &b, const TcS
     if (npx <= 0)
         return cudaSuccess;
     switch (k.test) {
-    case 0:
-        e = cudaFuncSetAttribute(tc_shp_pair_kernel<0>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    case 0: {
+        const size_t bytes = sizeof(float) * wpb * tc_ks_floats(s.n, s.area);
+
+        e = cudaFuncSetAttribute(tc_shp_ks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bytes);
         if (e == cudaSuccess)
-            tc_shp_pair_kernel<0><<<blocks, threads, smem, st>>>(s, b, k, amp, valid, logstat,
-                                                                 mask, vec);
+            tc_shp_ks_kernel<<<blocks, threads, bytes, st>>>(s, b, k, amp, valid, mask, vec > 1);
         break;
+    }
     case 1:
         e = cudaFuncSetAttribute(tc_shp_pair_kernel<1>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

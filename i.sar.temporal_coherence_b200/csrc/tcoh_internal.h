@@ -232,6 +232,9 @@ cudaError_t tc_launch_shp(const TcStrip &s, const TcChunk &c, const TcShpConst &
 struct TcShpBlock {
     int row0, nrows, crows, tiles_x;
     long long chunk_words;
+    /* ceil(2^32 / d) of the window's columns and of crows (0 for d = 1), set at
+       the launch: the kernels divide by these once per pair */
+    unsigned wr_magic, crows_magic;
 };
 
 /* SHP masks and counts of a block of chunks with every unordered pair of

@@ -57,3 +57,19 @@ def test_two_warp_kernel_far_scales(scale):
     """Sums beyond the branch-free quotients' range take the general form."""
     compare(35, 17, 9, scale=scale, window=(21, 7), shp_test="ks", alpha=0.01, min_shp=20,
             estimator="evd", bias=True)
+
+
+def test_two_dates_with_a_binding_ks_threshold():
+    """Two dates make one staged pair per candidate; alpha = 0.9 puts ks_max
+    below n, so that the comparisons decide."""
+    compare(2, 19, 9, window=(21, 7), shp_test="ks", alpha=0.9, min_shp=20, estimator="evd",
+            bias=False)
+
+
+@pytest.mark.parametrize("window", [(1, 7), (21, 1), (3, 3)])
+@pytest.mark.parametrize("shp_test", ["ks", "ad", "tlog"])
+def test_narrow_windows(window, shp_test):
+    """Windows of one row or one column (the pair kernels divide by their
+    sizes)."""
+    compare(3, 23, 17, window=window, shp_test=shp_test, alpha=0.05, min_shp=3,
+            estimator="evd", bias=False)
