@@ -595,58 +595,88 @@ __device__ bool ex_linked(int n, const ExWs &w)
    sweeping pivot k maps a_ij -> a_ij - a_ik a_kj / a_kk,
    a_ik, a_kj -> a_ik / a_kk, a_kk -> -1 / a_kk, and all pivots leave
    -A^-1, negated back at the end. It takes indefinite matrices. False when
-   a pivot's magnitude is not above floor_ (A is then undefined).
-   Each step copies the next pivot row as it updates it (into one of two
-   buffers), so that one barrier a pivot suffices; against a form that
-   scaled the pivot row into its own buffer behind a second barrier, this
-   one is the faster at every size (30-date AD/EMI/-b exact tier 83.7 ->
-   82.0 ms per 4096 x 4096 step). */
-__device__ bool ex_sweep(int n, int npu, const ExWs &w, double *A, double floor_)
+   a pivot's magnitude is not above floor_ (A is then as it was).
+
+   The matrix is in registers, TPR threads per row: thread h of a row has the
+   columns c = h mod TPR, in the order of the pivots to come (register q: column
+   TPR (shift + q) + h), so that pivot k is register 0 of the threads h = k mod
+   TPR, with static indices, and TPR pivots make one shift of the registers.
+   Those threads publish the pivot column, which is the pivot row (the matrix
+   stays symmetric), in the order in which each thread reads its part; the next
+   column goes out as soon as it is updated, into the other of two buffers, so
+   that one barrier a pivot suffices. With the packed triangle in shared memory
+   every update came with four shared accesses and its index arithmetic: 297
+   thousand cycles a pixel at 60 dates, 50 thousand now (63 and 24 at 30); the
+   link stage of 40 x 1024 pixels at 60 dates, EMI, 37.4 -> 27.8 ms. */
+template <int TPR>
+__device__ bool ex_sweep(int n, const ExWs &w, double *A, double floor_)
 {
-    const int t = threadIdx.x;
-    /* the pivot row as it stands before its step, in one of two buffers
-       (w.lu, free until the eigenvector): the step that updates row kp + 1
-       also copies it to the other buffer, so that one barrier a pivot
-       suffices */
-    double *raw[2] = {w.lu, w.lu + 64};
+    constexpr int NR = EX_THREADS / TPR, CP = NR / TPR; /* rows; columns per thread */
+    constexpr int PS = CP + 2; /* parts 16 bytes apart modulo the banks */
+    const int t = threadIdx.x, i = t / TPR, h = t % TPR;
+    double g[CP];
+    int shift = 0;
+    /* place of row i's entry in a buffer */
+    auto place = [&](int sh) { return (i % TPR) * PS + ((i / TPR - sh) & (CP - 1)); };
 
-    for (int j = t; j < n; j += EX_THREADS)
-        raw[0][j] = A[ex_sym(n, 0, j)];
-    __syncthreads();
-    for (int kp = 0; kp < n; kp++) {
-        const double *rk = raw[kp & 1];
-        double *rn = raw[(kp + 1) & 1];
-        const double d = rk[kp];
+#pragma unroll
+    for (int q = 0; q < CP; q++) {
+        const int c = TPR * q + h;
 
-        if (!(fabs(d) > floor_)) {
-            __syncthreads();
-            return false;
-        }
-        const double id = ex_rcp_any(d);
-
-        for (int q = t; q < npu; q += EX_THREADS) {
-            const int i = w.tab[q] >> 8, j = w.tab[q] & 255;
-            const double ri = rk[i] * id, rj = rk[j] * id;
-            double a;
-
-            if (i == kp && j == kp)
-                a = -id;
-            else if (i == kp)
-                a = rj;
-            else if (j == kp)
-                a = ri;
-            else
-                a = fma(-ri * d, rj, A[q]);
-            A[q] = a;
-            if (i == kp + 1)
-                rn[j] = a;
-            else if (j == kp + 1)
-                rn[i] = a;
-        }
-        __syncthreads();
+        g[q] = i < n && c < n ? A[ex_sym(n, i, c)] : 0.0;
     }
-    for (int q = t; q < npu; q += EX_THREADS)
-        A[q] = -A[q];
+    if (h == 0)
+        w.lu[place(0)] = g[0];
+    __syncthreads();
+#pragma unroll 1
+    for (int base = 0; base < n; base += TPR) {
+#pragma unroll
+        for (int s = 0; s < TPR; s++) {
+            const int k = base + s;
+
+            if (k >= n)
+                break;
+            const double *r = w.lu + TPR * PS * (k & 1);
+            double *rn = w.lu + TPR * PS * ((k + 1) & 1);
+            const double d = r[s * PS];
+
+            if (!(fabs(d) > floor_)) {
+                __syncthreads();
+                return false;
+            }
+            const double id = ex_rcp_any(d);
+            /* the pivot row scales by 1 / a_kk: a_kj - (1 - 1 / a_kk) a_kj */
+            const double f = i == k ? 1.0 - id : r[place(shift)] * id;
+            auto update = [&](int q) { g[q] = fma(-f, r[h * PS + q], g[q]); };
+
+            update(0);
+            update(1);
+            if (h == (s + 1) % TPR)
+                rn[place(shift + (s + 1 == TPR))] = s + 1 == TPR ? g[1] : g[0];
+#pragma unroll
+            for (int q = 2; q < CP; q++)
+                update(q);
+            if (h == s)
+                g[0] = i == k ? -id : f;
+            if (s + 1 == TPR) {
+                const double g0 = g[0];
+
+#pragma unroll
+                for (int q = 0; q < CP - 1; q++)
+                    g[q] = g[q + 1];
+                g[CP - 1] = g0;
+                shift++;
+            }
+            __syncthreads();
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < CP; q++) {
+        const int c = TPR * ((shift + q) & (CP - 1)) + h;
+
+        if (i <= c && c < n)
+            A[tc_pidx(n, i, c)] = -g[q];
+    }
     __syncthreads();
     return true;
 }
@@ -768,11 +798,12 @@ __device__ bool ex_gauss_jordan(int n, const ExWs &w, double *A)
    dates; in the CTA's global scratch W above); else, or when the inverse is
    not moderate, the Jacobi eigen-pseudo-inverse with the absolute floor
    1e-9 (tests/reference.py:151-156) on warp 0. Returns status bits. */
+template <int TPR>
 __device__ unsigned ex_inverse(int n, int npu, int ld, const ExWs &w, double *W)
 {
     const int t = threadIdx.x;
 
-    if (ex_sweep(n, npu, w, w.G, 1.0e-5) && ex_moderate(n, npu, w, w.G))
+    if (ex_sweep<TPR>(n, w, w.G, 1.0e-5) && ex_moderate(n, npu, w, w.G))
         return 0;
     double *A = n <= 32 ? (double *)w.stage : W;
 
@@ -1532,7 +1563,7 @@ tc_link_exact_kernel(TcStrip s, TcChunk c, TcLinkConst k, ExLayout L,
         unsigned st = TC_STATUS_FP64;
 
         if (k.emi) {
-            st |= ex_inverse(n, npu, ld, w, W);
+            st |= ex_inverse<(NB > 1 ? 2 : 4)>(n, npu, ld, w, W);
             /* M = |T|^-1 o T in place of T; T in float in place of |T|^-1 */
             for (int q = t; q < npu; q += EX_THREADS) {
                 const double g = w.G[q];

@@ -1,7 +1,8 @@
 """The link kernels at the edges of their ranges of dates (B200 only): the
 half-warp kernel's padded rows and columns (up to 32 dates) and the two-warp
 kernel's blocks of eight columns, its second warp's last rows and its pixels per
-CTA (33 to 64 dates), against the double-precision oracle."""
+CTA (33 to 64 dates), the double-precision tier's rows and columns in registers,
+against the double-precision oracle."""
 
 import numpy as np
 import pytest
@@ -50,6 +51,14 @@ def test_half_warp_kernel(n, estimator):
 def test_two_warp_kernel(n, bias):
     compare(n, 18, 7, window=(21, 7), shp_test="ks", alpha=0.01, min_shp=20, estimator="evd",
             bias=bias)
+
+
+@pytest.mark.parametrize("n", [3, 5, 29, 32, 33, 34, 40, 63, 64])
+def test_exact_tier_emi(n):
+    """EMI in double precision: every pixel above 32 dates, below it the pixels
+    that the bias correction's threshold sends there."""
+    compare(n, 18, 7, window=(21, 7), shp_test="ks", alpha=0.01, min_shp=20, estimator="emi",
+            bias=True)
 
 
 @pytest.mark.parametrize("scale", [3.0e-12, 3.0e11])
