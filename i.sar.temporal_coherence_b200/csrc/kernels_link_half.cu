@@ -2364,7 +2364,7 @@ size_t tc_link_half_scratch_bytes(int n, int sms)
 {
     /* EMI only, per group (two per warp, at most 8 warps per CTA, one CTA
        per SM): |T|, the Jacobi eigenvectors and eigenvalues of the fallback
-       tiers. Stacks of more than 32 dates take the shared-memory kernel. */
+       tiers. Stacks of more than 32 dates take other kernels. */
     if (n > 32)
         return 256;
     return (size_t)sms * 16 * (2 * n * (n | 1) + 32) * sizeof(double);
