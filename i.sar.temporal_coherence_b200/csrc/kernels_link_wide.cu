@@ -13,8 +13,8 @@
  * pixels at 60 dates, a Householder step 0.55k cycles per pixel instead of 0.78k.
  *
  * Bound by latency: a step's reductions, barriers and shared-memory round trips
- * (short scoreboard) with three warps per scheduler, a third of the issue slots
- * in use. With the matrix itself in shared memory (a warp per pixel, twelve
+ * (short scoreboard) with three warps per scheduler, half of the issue slots in
+ * use. With the matrix itself in shared memory (a warp per pixel, twelve
  * pixels per SM) each multiply-add came with its own loads and stores of the
  * matrix and a step's serial work was done by one lane: 55.8 ms on the same
  * pixels, 6.29 against 4.25 ms on 61 x 517 at 45 dates.
