@@ -19,7 +19,10 @@
  */
 #include "tcoh_internal.h"
 
+#include <limits.h>
 #include <math.h>
+
+#include <type_traits>
 
 /* AoS [npad][N] float2 -> SoA [planes][npad] float2, zero planes >= N. */
 __global__ void tc_prep_kernel(TcStrip s, const float2 *__restrict__ aos,
@@ -543,6 +546,14 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
     }
 }
 
+/* Shared floats per warp of tc_shp_ks_kernel, a multiple of 4. */
+__host__ __device__ inline int tc_ks_floats(int n, int area, bool far)
+{
+    const int n4 = (n + 3) & ~3;
+
+    return 2 * n4 + ((32 * (n | 1) + 4 + (far ? 64 : 32) + (area + 1) / 2 + 3) & ~3);
+}
+
 /* KS without the merge walk. With both series sorted, the walk's largest
    |ia - ib| stays within m = ks_max exactly when (centre a first on ties)
        b[i - m] < a[i]  and  a[i - m] <= b[i]   for all i >= m:
@@ -559,21 +570,26 @@ tc_shp_pair_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restric
    walk's 10 per step and two steps per value, bound by instruction issue as that
    was: SHP stage 1.37 -> 0.86 ms on 250 x 1000 pixels at 30 dates, 2.33 -> 1.37
    ms on 96 x 2048 at 60, 0.69 -> 0.54 ms on 512 x 512 at 10 (there the lists of
-   candidates and the bits set for the other pixel weigh as much). */
+   candidates and the bits set for the other pixel weigh as much).
+
+   FAR: the window spans 2^31 amplitudes or more, and the candidates' places are
+   64-bit (with whole addresses at every size, a call on 512 x 512 pixels at 10
+   dates took 1.88 ms instead of 1.84). */
+template <bool FAR>
 __global__ void __launch_bounds__(256)
 tc_shp_ks_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restrict__ amp,
                  const unsigned char *__restrict__ valid, uint32_t *__restrict__ mask, int pair)
 {
     extern __shared__ float4 sm4[];
+    using Place = typename std::conditional<FAR, long long, int>::type;
     const int n = s.n, n4 = (n + 3) & ~3, ld = n | 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
-    /* floats per warp, a multiple of 4: see tc_ks_floats */
-    const int per_warp = 2 * n4 + ((32 * ld + 4 + 32 + (s.area + 1) / 2 + 3) & ~3);
+    const int per_warp = tc_ks_floats(n, s.area, FAR);
     float *lo = (float *)sm4 + warp * per_warp; /* a[j - m] */
     float *hi = lo + n4;                        /* a[j + m] */
     float *stage = hi + n4;                     /* 32 rows of ld, 4 to spare */
-    int *rel = (int *)(stage + 32 * ld + 4);    /* the candidates' places */
+    Place *rel = (Place *)(stage + 32 * ld + 4); /* the candidates' places */
     unsigned short *list = (unsigned short *)(rel + 32);
     const int cc = (s.wa / 2) * s.wr + s.wr / 2; /* the centre's own index */
     const long long npx = (long long)b.nrows * s.cols;
@@ -627,7 +643,7 @@ tc_shp_ks_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restrict_
             const int dy = div_magic(c, s.wr, b.wr_magic), dx = c - dy * s.wr;
 
             /* an idle lane's row: candidate 0's, inside the strip */
-            rel[lane] = (dy * s.W + dx) * n;
+            rel[lane] = ((Place)dy * s.W + dx) * n;
             __syncwarp();
             if (pair) {
 #pragma unroll 5
@@ -691,14 +707,6 @@ tc_shp_ks_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restrict_
     }
 }
 
-/* Shared floats per warp of tc_shp_ks_kernel. */
-static int tc_ks_floats(int n, int area)
-{
-    const int n4 = (n + 3) & ~3;
-
-    return 2 * n4 + ((32 * (n | 1) + 4 + 32 + (area + 1) / 2 + 3) & ~3);
-}
-
 /* SHP counts of the block's output pixels from their masks; -1 for an
    invalid centre. */
 __global__ void tc_shp_count_kernel(TcStrip s, TcShpBlock b, const unsigned char *__restrict__ valid,
@@ -744,12 +752,13 @@ cudaError_t tc_launch_shp_block(const TcStrip &s, const TcShpBlock &blk, const T
         return cudaSuccess;
     switch (k.test) {
     case 0: {
-        const size_t bytes = sizeof(float) * wpb * tc_ks_floats(s.n, s.area);
+        const bool far = ((long long)(s.wa - 1) * s.W + s.wr) * s.n > INT_MAX;
+        const size_t bytes = sizeof(float) * wpb * tc_ks_floats(s.n, s.area, far);
+        auto kernel = far ? tc_shp_ks_kernel<true> : tc_shp_ks_kernel<false>;
 
-        e = cudaFuncSetAttribute(tc_shp_ks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)bytes);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e == cudaSuccess)
-            tc_shp_ks_kernel<<<blocks, threads, bytes, st>>>(s, b, k, amp, valid, mask, vec > 1);
+            kernel<<<blocks, threads, bytes, st>>>(s, b, k, amp, valid, mask, vec > 1);
         break;
     }
     case 1:
