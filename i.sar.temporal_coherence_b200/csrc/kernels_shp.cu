@@ -593,7 +593,9 @@ tc_shp_ks_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restrict_
     unsigned short *list = (unsigned short *)(rel + 32);
     const int cc = (s.wa / 2) * s.wr + s.wr / 2; /* the centre's own index */
     const long long npx = (long long)b.nrows * s.cols;
-    const int m = k.ks_max;
+    /* below 0 no series passes, the centre's own included */
+    const bool any = k.ks_max >= 0;
+    const int m = max(k.ks_max, 0);
     /* elements of the staging loop: single values, or pairs where every series
        starts on 8 bytes */
     const int nu = pair ? n / 2 : n;
@@ -665,7 +667,7 @@ tc_shp_ks_kernel(TcStrip s, TcShpBlock b, TcShpConst k, const float *__restrict_
             }
             __syncwarp();
             const float *row = stage + lane * ld;
-            bool fwd = act, rev = act;
+            bool fwd = act && any, rev = act && any;
 
             /* places from n on: NaN against whatever follows the row */
 #pragma unroll 2

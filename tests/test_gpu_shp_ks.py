@@ -56,6 +56,25 @@ def test_tied_amplitudes(n, levels):
         assert np.array_equal(got, walk_counts(amp, valid, rows, cols, window, m)), m
 
 
+@pytest.mark.parametrize("m", [-1, -5, -2**31, 2**31 - 1])
+def test_thresholds_out_of_range(m):
+    """Settings may hold any threshold: below 0 nothing passes, from n on all."""
+    n, rows, cols = 6, 9, 8
+    rng = np.random.default_rng(1)
+    amp = np.sort(rng.uniform(1, 2, (rows, cols, n)).astype(np.float32), axis=2)
+    valid = np.ones((rows, cols), np.uint8)
+    slc = np.stack([amp, amp], axis=3)
+    for window in ((1, 1), (5, 3)):
+        s = tcoh_b200.make_settings(n, window=(5, 3), shp_test="ks", min_shp=6)
+        s.win_az, s.win_rg, s.ks_max = window + (m,)
+        r, c = rows - window[0] + 1, cols - window[1] + 1
+        with tcoh_b200.Backend(s, cols) as be:
+            got = be.run(slc, amp, valid, r, c)
+        assert (got["count"] == (0 if m < 0 else window[0] * window[1])).all()
+        if m < 0:
+            assert np.isnan(got["coh"]).all()
+
+
 def test_window_of_more_than_2_31_amplitudes():
     """1001 x 1 candidates, 33,600 columns, 64 dates: the last rows' candidates
     lie 2^31 amplitudes and more beyond the first (52 GB of device memory). With
