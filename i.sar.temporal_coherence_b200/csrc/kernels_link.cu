@@ -17,7 +17,7 @@
  * from a Gram kernel's sums, handing the pixels that need it to the exact tier;
  * EMI of 33 to 64 dates is all exact tier.
  */
-#include "tcoh_internal.h"
+#include "link_float.cuh"
 
 #include <math.h>
 
@@ -1443,21 +1443,12 @@ __device__ float ex_gamma(int n, int npu, const ExWs &w)
 
         if (i == j)
             continue;
-        const float2 tv = w.Tf[q];
-        const float m2 = tv.x * tv.x + tv.y * tv.y;
-        float ur = 1.f, ui = 0.f;
-
-        if (m2 > 0.f) {
-            const float r = rsqrtf(m2);
-
-            ur = tv.x * r;
-            ui = tv.y * r;
-        }
+        const float2 u = unit_phasor(w.Tf[q]);
         const float2 zi = w.zs[i], zj = w.zs[j];
         const float wr = zi.x * zj.x + zi.y * zj.y, wi = zi.x * zj.y - zi.y * zj.x;
 
-        sr += ur * wr - ui * wi;
-        si += ur * wi + ui * wr;
+        sr += u.x * wr - u.y * wi;
+        si += u.x * wi + u.y * wr;
     }
     const double2 ssum = ex_sum2(sr, si, w.red);
 

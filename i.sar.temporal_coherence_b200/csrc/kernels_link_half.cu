@@ -1653,22 +1653,13 @@ __device__ float gamma16(int n, int ld, const HWs &w, const Pair &g, double2 z0d
 
         if (i == j)
             continue;
-        const float2 tv = w.T[i * ld + j];
-        const float m2 = tv.x * tv.x + tv.y * tv.y;
-        float ur = 1.f, ui = 0.f;
-
-        if (m2 > 0.f) {
-            const float r = rsqrt_approx(m2);
-
-            ur = tv.x * r;
-            ui = tv.y * r;
-        }
+        const float2 u = unit_phasor(w.T[i * ld + j]);
         const float2 zi = w.zs[i], zj = w.zs[j];
         const float wr = zi.x * zj.x + zi.y * zj.y;
         const float wi = zi.x * zj.y - zi.y * zj.x;
 
-        sr += ur * wr - ui * wi;
-        si += ur * wi + ui * wr;
+        sr += u.x * wr - u.y * wi;
+        si += u.x * wi + u.y * wr;
     }
     sr = gsum(sr, g);
     si = gsum(si, g);

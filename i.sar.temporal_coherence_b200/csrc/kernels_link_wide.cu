@@ -791,14 +791,11 @@ __device__ float goodness(int n, int ld, const Ws &w, const Duo &g, float2 z,
 #pragma unroll 4
     for (int q = i; q < npu; q += 64) {
         const int a = upper_tab[q] >> 8, b = upper_tab[q] & 255;
-        const float2 tv = w.T[a * ld + b], za = w.z[a], zb = w.z[b];
-        const float m2 = tv.x * tv.x + tv.y * tv.y;
-        const float s = m2 > 0.f ? rsqrtf(m2) : 0.f;
-        const float ur = m2 > 0.f ? tv.x * s : 1.f, ui = tv.y * s;
+        const float2 u = unit_phasor(w.T[a * ld + b]), za = w.z[a], zb = w.z[b];
         const float wr = za.x * zb.x + za.y * zb.y, wi = za.x * zb.y - za.y * zb.x;
 
-        sr += a == b ? 0.f : ur * wr - ui * wi;
-        si += a == b ? 0.f : ur * wi + ui * wr;
+        sr += a == b ? 0.f : u.x * wr - u.y * wi;
+        si += a == b ? 0.f : u.x * wi + u.y * wr;
     }
     sr = wsum(sr);
     si = wsum(si);

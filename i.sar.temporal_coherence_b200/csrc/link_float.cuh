@@ -7,6 +7,8 @@
 
 #include "tcoh_internal.h"
 
+#include <float.h>
+
 /* A value that the compiler cannot follow: the addresses formed from it are
    not kept in registers from one pixel pair to the next (there are more of
    them than registers; they would be spilled). */
@@ -59,6 +61,21 @@ __device__ __forceinline__ float sqrt_rn(float a)
     h = fmaf(h, e, h);
     s = fmaf(s, e, s);
     return fmaf(fmaf(-s, s, a), h, s);
+}
+
+/* T_ij / |T_ij| of the goodness of fit (tcoh.cl:734-738); 1 for |T_ij| below
+   1e-37 (|T_ij| is at most 1). The factor 2^60, which changes no rounding, keeps
+   the square normal: without it the approximate root flushed the square of
+   |T_ij| < 1.1e-19 (dates whose energy lies in different pixels) to zero, and the
+   phasor was infinite. */
+__device__ __forceinline__ float2 unit_phasor(float2 t)
+{
+    const float x = t.x * 0x1p60f, y = t.y * 0x1p60f;
+    const float m2 = x * x + y * y;
+    const bool some = m2 >= FLT_MIN;
+    const float s = some ? rsqrt_approx(m2) : 0.f;
+
+    return make_float2(some ? x * s : 1.f, y * s);
 }
 
 /* Fused products with the roundings written out, so that what a pixel gets does
