@@ -188,8 +188,7 @@ cudaError_t tc_launch_adjoint_scatter(const TcStrip &s, const TcChunk &c, int ha
                                       const float *slc, float *dtheta, cudaStream_t st)
 {
     const int bytes = TC_TILE_PIX * GS_LD * 8 + s.wa * TC_TILE_PIX * 4;
-    cudaError_t e = cudaFuncSetAttribute(tc_adjoint_scatter_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = tc_allow_smem(tc_adjoint_scatter_kernel);
 
     if (e != cudaSuccess)
         return e;

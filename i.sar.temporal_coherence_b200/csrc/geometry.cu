@@ -469,8 +469,7 @@ cudaError_t launch_prep_raw(unsigned blocks, int n, const float *re, const float
                             cudaStream_t st)
 {
     const int bytes = 8 * 32 * (n | 1) * (int)sizeof(float2);
-    cudaError_t e = cudaFuncSetAttribute(tc_prep_raw_kernel<NP>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = tc_allow_smem(tc_prep_raw_kernel<NP>);
 
     if (e != cudaSuccess)
         return e;

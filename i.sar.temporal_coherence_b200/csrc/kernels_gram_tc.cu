@@ -860,8 +860,7 @@ cudaError_t tc_launch_gram_tensor(const TcStrip &s, const TcChunk &c, int split_
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    if ((e = cudaFuncSetAttribute(tc_gram_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  bytes)) != cudaSuccess)
+    if ((e = tc_allow_smem(tc_gram_tc_kernel)) != cudaSuccess)
         return e;
     /* persistent: two CTAs per SM (the TMEM of two accumulators) */
     const int grid = items < 2 * sms ? items : 2 * sms;
@@ -897,11 +896,9 @@ cudaError_t tc_launch_adjoint_scatter_tensor(const TcStrip &s, const TcChunk &c,
                                              const float *slc, float *dtheta, cudaStream_t st)
 {
     const AdjSmem L = adj_smem(s.wa);
-    cudaError_t e;
+    const cudaError_t e = tc_allow_smem(tc_gram_adjoint_tc_kernel);
 
-    if ((e = cudaFuncSetAttribute(tc_gram_adjoint_tc_kernel,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes)) !=
-        cudaSuccess)
+    if (e != cudaSuccess)
         return e;
     tc_gram_adjoint_tc_kernel<<<c.npix / TC_TILE_PIX, ADJ_THREADS, L.bytes, st>>>(
         s, c, halo, gbar, mask, (const float2 *)slc, dtheta);

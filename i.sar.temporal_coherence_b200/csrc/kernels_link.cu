@@ -1615,8 +1615,7 @@ static cudaError_t launch_exact_nb(const TcStrip &s, const TcChunk &c, const TcL
         blocks = c.npix;
     if (q && q->pending < ctas)
         blocks = (int)q->pending;
-    cudaError_t e = cudaFuncSetAttribute(tc_link_exact_kernel<NB, BC>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes);
+    const cudaError_t e = tc_allow_smem(tc_link_exact_kernel<NB, BC>);
 
     if (e != cudaSuccess)
         return e;

@@ -2375,7 +2375,7 @@ static cudaError_t launch_half(const TcStrip &s, const TcChunk &c, const TcLinkC
     const size_t per_warp = 2 * (size_t)L.per_group;
     const size_t tab = ((size_t)tc_npu(s.n) * 2 + 15) & ~(size_t)15;
     const int max_warps = half_warps(EMI, ADJ);
-    int wpb = (int)((227 * 1024 - tab) / per_warp);
+    int wpb = (int)((TC_SMEM_MAX - tab) / per_warp);
 
     if (wpb > max_warps)
         wpb = max_warps;
@@ -2390,8 +2390,7 @@ static cudaError_t launch_half(const TcStrip &s, const TcChunk &c, const TcLinkC
     const size_t smem = per_warp * wpb + tab;
     const int want = (c.npix / 2 + wpb - 1) / wpb;
     const int blocks = want < sms ? want : sms;
-    cudaError_t e = cudaFuncSetAttribute(tc_link_half_kernel<EMI, ADJ>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = tc_allow_smem(tc_link_half_kernel<EMI, ADJ>);
 
     if (e != cudaSuccess)
         return e;

@@ -926,7 +926,7 @@ cudaError_t tc_launch_link_wide(const TcStrip &s, const TcChunk &c, const TcLink
 {
     const WideLayout L = wide_layout(s.n);
     const size_t tab = ((size_t)tc_npu(s.n) * 2 + 15) & ~(size_t)15;
-    int pixels = (int)((227 * 1024 - tab) / L.per_pixel);
+    int pixels = (int)((TC_SMEM_MAX - tab) / L.per_pixel);
 
     if (pixels > WD_PIXELS)
         pixels = WD_PIXELS;
@@ -936,8 +936,7 @@ cudaError_t tc_launch_link_wide(const TcStrip &s, const TcChunk &c, const TcLink
     const size_t smem = (size_t)pixels * L.per_pixel + tab;
     const int want = (c.npix + pixels - 1) / pixels;
     const int blocks = want < sms ? want : sms;
-    const cudaError_t e = cudaFuncSetAttribute(
-        tc_link_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = tc_allow_smem(tc_link_wide_kernel);
 
     if (e != cudaSuccess)
         return e;

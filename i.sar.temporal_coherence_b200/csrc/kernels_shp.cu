@@ -280,22 +280,19 @@ cudaError_t tc_launch_shp(const TcStrip &s, const TcChunk &c, const TcShpConst &
 
     switch (k.test) {
     case 0:
-        e = cudaFuncSetAttribute(tc_shp_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
+        e = tc_allow_smem(tc_shp_kernel<0>);
         if (e == cudaSuccess)
             tc_shp_kernel<0><<<blocks, threads, smem, st>>>(s, c, k, amp, valid, logstat, mask,
                                                             count, vec);
         break;
     case 1:
-        e = cudaFuncSetAttribute(tc_shp_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
+        e = tc_allow_smem(tc_shp_kernel<1>);
         if (e == cudaSuccess)
             tc_shp_kernel<1><<<blocks, threads, smem, st>>>(s, c, k, amp, valid, logstat, mask,
                                                             count, vec);
         break;
     default:
-        e = cudaFuncSetAttribute(tc_shp_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
+        e = tc_allow_smem(tc_shp_kernel<2>);
         if (e == cudaSuccess)
             tc_shp_kernel<2><<<blocks, threads, smem, st>>>(s, c, k, amp, valid, logstat, mask,
                                                             count, vec);
@@ -758,21 +755,19 @@ cudaError_t tc_launch_shp_block(const TcStrip &s, const TcShpBlock &blk, const T
         const size_t bytes = sizeof(float) * wpb * tc_ks_floats(s.n, s.area, far);
         auto kernel = far ? tc_shp_ks_kernel<true> : tc_shp_ks_kernel<false>;
 
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        e = tc_allow_smem(kernel);
         if (e == cudaSuccess)
             kernel<<<blocks, threads, bytes, st>>>(s, b, k, amp, valid, mask, vec > 1);
         break;
     }
     case 1:
-        e = cudaFuncSetAttribute(tc_shp_pair_kernel<1>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = tc_allow_smem(tc_shp_pair_kernel<1>);
         if (e == cudaSuccess)
             tc_shp_pair_kernel<1><<<blocks, threads, smem, st>>>(s, b, k, amp, valid, logstat,
                                                                  mask, vec);
         break;
     default:
-        e = cudaFuncSetAttribute(tc_shp_pair_kernel<2>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = tc_allow_smem(tc_shp_pair_kernel<2>);
         if (e == cudaSuccess)
             tc_shp_pair_kernel<2><<<blocks, threads, smem, st>>>(s, b, k, amp, valid, logstat,
                                                                  mask, vec);

@@ -18,6 +18,22 @@
 #define TC_TILE_W 8
 #define TC_TILE_PIX (TC_TILE_H * TC_TILE_W)
 
+/* Shared memory that a CTA can have. */
+constexpr int TC_SMEM_MAX = 227 * 1024;
+
+#ifdef __CUDACC__
+/* Lets the launches of a kernel take up to TC_SMEM_MAX of dynamic shared memory.
+   The limit belongs to the function on a device, not to the launch that it is
+   raised for: all callers set the same one, whatever they take, so that contexts
+   on several host threads cannot lower it under one another between the call and
+   the launch. */
+template <class Kernel>
+inline cudaError_t tc_allow_smem(Kernel *kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX);
+}
+#endif
+
 /* Per-strip constants. */
 struct TcStrip {
     int n;           /* dates */
