@@ -821,10 +821,10 @@ __device__ __forceinline__ double rcp_newton(double d)
    symmetric, pivot row k is assembled from every lane's own column-k
    entries. The register columns rotate by one per step so that the pivot
    column is always g[0] (the step loop stays a run-time loop): on return
-   register column p holds true column (p + n) & 31. Each step updates the
+   register column p holds true column (p + n) mod NC. Each step updates the
    next pivot column first and publishes it, so that the next pivot's
    reciprocal (a chain of eight dependent operations) forms while the other
-   columns update. rs holds 3 x 32 doubles, taken in turn: a step writes the
+   columns update. rs holds 3 x NC doubles, taken in turn: a step writes the
    buffer that was last read before the barrier of the step before it. False
    when a pivot's magnitude is not above `floor`. */
 template <class G>
@@ -832,7 +832,7 @@ __device__ bool sweep16(double (&g0)[NC], double (&g1)[NC], int n, double floor,
                         const G &g)
 {
     const int i0 = g.gl, i1 = g.gl + 16;
-    /* a_ik, in the order of the registers: r[p] = a_k,(p + k) & 31 */
+    /* a_ik, in the order of the registers: r[p] = a_k,(p + k) mod NC */
     double *r = rs;
 
     r[i0] = g0[0];
@@ -2022,6 +2022,15 @@ constexpr int half_warps(bool emi, bool adj)
     return TWO ? (emi || adj ? 8 : 12) : (emi ? 16 : 24);
 }
 
+/* Scratch slots per CTA of EMI's fallback tiers: one per group with two rows per
+   lane; one per warp, its halves in turn, with one row per lane and twice the
+   warps. */
+constexpr int HALF_SLOTS = 16;
+
+static_assert(half_warps(true, false) * (TWO ? 2 : 1) <= HALF_SLOTS &&
+                  half_warps(true, true) * (TWO ? 2 : 1) <= HALF_SLOTS,
+              "a slot per group or warp");
+
 /* ADJ: after gamma, backward16 writes the gradient of gamma with respect
    to the pixel's coherence sums into gbar (same layout as gram). */
 template <bool EMI, bool ADJ>
@@ -2043,8 +2052,7 @@ tc_link_half_kernel(TcStrip s, TcChunk c, TcLinkConst k, HalfLayout L,
     const HWs w = hws(smem + (size_t)grp * L.per_group, L);
     const int n = s.n, ld = L.ld;
     const long long plane = (long long)s.rows * s.cols;
-    /* EMI's fallback tiers: a slot per group, or (one row per lane, more warps)
-       per warp, its halves in turn; 16 per CTA either way */
+    /* EMI's fallback tiers, see HALF_SLOTS */
     double *V = scratch + (TWO ? (size_t)blockIdx.x * wpb * 2 + grp
                                : (size_t)blockIdx.x * wpb + warp) * (size_t)(2 * n * ld + 32);
     const int i0 = g.gl, i1 = g.gl + 16;
@@ -2353,12 +2361,12 @@ HalfLayout half_layout(int n, int emi, int adj = 0)
 #if TC_LINK_COLS == 32
 size_t tc_link_half_scratch_bytes(int n, int sms)
 {
-    /* EMI only, per group (two per warp, at most 8 warps per CTA, one CTA
-       per SM): |T|, the Jacobi eigenvectors and eigenvalues of the fallback
-       tiers. Stacks of more than 32 dates take other kernels. */
+    /* EMI only, per slot (HALF_SLOTS per CTA, one CTA per SM): |T|, the Jacobi
+       eigenvectors and eigenvalues of the fallback tiers. Stacks of more than 32
+       dates take other kernels. */
     if (n > 32)
         return 256;
-    return (size_t)sms * 16 * (2 * n * (n | 1) + 32) * sizeof(double);
+    return (size_t)sms * HALF_SLOTS * (2 * n * (n | 1) + 32) * sizeof(double);
 }
 #endif
 
@@ -2380,7 +2388,7 @@ static cudaError_t launch_half(const TcStrip &s, const TcChunk &c, const TcLinkC
     if (wpb > max_warps)
         wpb = max_warps;
     /* few pixels: over all SMs rather than in full CTAs on some (a 48 x 40 crop
-       at 10 dates: 33 -> 21 us) */
+       at 10 dates: 31 -> 21 us, with one row per lane) */
     const int spread = ((c.npix + 1) / 2 + sms - 1) / sms;
 
     if (wpb > spread)
