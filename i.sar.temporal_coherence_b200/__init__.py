@@ -496,10 +496,16 @@ def temporal_coherence(stack, window=(21, 7), shp_test="ks", alpha=0.05, min_shp
         # took 23 of the 40 ms of a 30 x 200 x 300 stack). Where the raw rows
         # would take a noticeable part of the device memory that the strip was
         # sized for, or the caller's context has a geometry of its own,
-        # read_strip prepares it.
+        # read_strip prepares it; also where the strip is small, and two more
+        # buffers and a copy per row block cost more than read_strip (by host
+        # and on the device, 60 dates, 40 x 40: 7.1 and 7.6 ms; 20 dates, 60 x
+        # 60: 6.1 and 6.7, 80 x 80: 8.1 and 7.2; 10 dates, 80 x 80: 6.1 and
+        # 6.6, 120 x 120: 8.5 and 7.5).
+        cells = (strip_rows + 2 * halo_az) * ncols
+        large = cells >= 12500 or cells >= 6500 and n * cells >= 140000
         raw = geometry is not None or (
-            phase is None and getattr(be, "_grid", None) is None
-            and 8 * n * (strip_rows + 2 * halo_az) * ncols <= be.max_alloc // 8)
+            phase is None and getattr(be, "_grid", None) is None and large
+            and 8 * n * cells <= be.max_alloc // 8)
         if raw:
             elev = None if elevation is None else np.asarray(elevation, np.float64)
         else:
