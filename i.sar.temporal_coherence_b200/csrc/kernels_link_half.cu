@@ -1025,10 +1025,11 @@ __device__ __forceinline__ int sym_idx(int n, int i, int j)
 /* |t| in double: the squares of the float parts are exact, their sum is
    rounded once; the root by two Newton steps (s += (m - s^2) / (2 s), in the
    form s += e h with h = 1 / (2 s) from the float reciprocal root, relative
-   error 2^-22 -> 2^-43 -> rounding), 0 below 3e-19. The library's root and
-   hypot branch, which keeps the entries of a batch from overlapping. ADJ:
-   hypot, within an ulp of it (the gradients of nearly degenerate pixels
-   magnify even that). */
+   error 2^-22 -> 2^-43 -> rounding), 0 below 3e-19 (such an entry's share of
+   M_ij, of the order of its square, is beneath M's float rounding). The
+   library's root and hypot branch, which keeps the entries of a batch from
+   overlapping. ADJ: hypot, within an ulp of it (the gradients of nearly
+   degenerate pixels magnify even that). */
 template <bool ADJ>
 __device__ __forceinline__ double abs_t(float2 t)
 {
